@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "dqb_small.cuh"
+#include "dqb_small_band.cuh"
 
 namespace dqb {
 
@@ -298,7 +299,8 @@ __global__ void __launch_bounds__(kSmallThreads, NP == 64 ? 1 : (NP == 32 ? 3 : 
     const long long pos = ctl.inst;
     if (pos >= a.batch) break;
     const long long inst = a.order ? (long long)a.order[pos] : pos;
-    if (inst < 0 || inst >= a.batch) {  // not a valid instance: skip it
+    // not a valid instance, or one that the banded kernel has solved: skip it
+    if (inst < 0 || inst >= a.batch || (a.pend && a.pend[inst * a.pend_stride] != band::kPending)) {
       __syncthreads();                    // every thread has read ctl.inst
       continue;
     }
@@ -464,6 +466,8 @@ static DenseSmallArgs make_args(const dqb_dense_problem* p, const dqb_ode_option
   a.Lidx = p->L_index;
   a.ridx = p->rho0_index;
   a.order = p->start_order;
+  a.pend = nullptr;
+  a.pend_stride = 0;
   a.states = out ? (float2*)out->states : nullptr;
   a.expects = out ? (float2*)out->expects : nullptr;
   a.infos = out ? out->infos : nullptr;
@@ -476,6 +480,24 @@ static DenseSmallArgs make_args(const dqb_dense_problem* p, const dqb_ode_option
   a.tape_y = nullptr;
   a.tape_cap = 0;
   return a;
+}
+
+// The instances with few nonzero diagonals first (hermitian form): the banded kernel, whose
+// work counter is the second word of the zeroed block at `counter`, marks the others in
+// their step counts for the product kernel that follows.
+static int solve_banded(DenseSmallArgs& a, unsigned int* counter, int feat, int tape_np, cudaStream_t s) {
+  if (a.o.form != DQB_FORM_HERMITIAN) return DQB_OK;
+  band::Args b;
+  b.d = a;
+  b.rag = nullptr;
+  b.counter = counter + 1;
+  b.pend = a.infos;
+  b.pend_stride = 3;
+  b.tape_np = tape_np;
+  if (int rc = band::run(b, a.n, feat, s)) return rc;
+  a.pend = a.infos;
+  a.pend_stride = 3;
+  return DQB_OK;
 }
 
 extern "C" int dqb_mesolve_dense(const dqb_dense_problem* p, const dqb_ode_options* o, const dqb_outputs* out,
@@ -498,6 +520,7 @@ extern "C" int dqb_mesolve_dense(const dqb_dense_problem* p, const dqb_ode_optio
   zero_words_kernel<<<1, 64, 0, s>>>((unsigned int*)workspace, 64);
   if (o->precision == DQB_PREC_F16X3 && small_tc_applies(p->n, p->n_jumps, o->form))
     return small_tc_launch(a, grid, s);
+  if ((rc = solve_banded(a, a.counter, 0, 0, s))) return rc;
   const size_t smem = smem_for(NP, p->n_jumps);
   switch (NP) {
     case 16: mesolve_small_kernel<16><<<grid, kSmallThreads, smem, s>>>(a); break;
@@ -560,6 +583,7 @@ extern "C" int dqb_mesolve_dense_td(const dqb_dense_problem* p, const dqb_td_ham
   a.td.n_jump = td->n_jump_ts;
   a.td.jump_ts = td->jump_ts;
   zero_words_kernel<<<1, 64, 0, s>>>((unsigned int*)workspace, 64);
+  if ((rc = solve_banded(a, a.counter, 1, 0, s))) return rc;
   const size_t smem = smem_for(NP, Keff);
   switch (NP) {
     case 16: mesolve_small_kernel<16, 1><<<grid, kSmallThreads, smem, s>>>(a); break;
@@ -925,6 +949,7 @@ extern "C" int dqb_mesolve_dense_taped(const dqb_dense_problem* p, const dqb_ode
   a.tape_y = (float2*)tape->y;
   a.tape_cap = tape->capacity;
   zero_words_kernel<<<1, 64, 0, s>>>((unsigned int*)workspace, 64);
+  if ((rc = solve_banded(a, a.counter, 2, NP, s))) return rc;
   const size_t smem = smem_for(NP, p->n_jumps);
   switch (NP) {
     case 16: mesolve_small_kernel<16, 2><<<grid, kSmallThreads, smem, s>>>(a); break;
@@ -1022,6 +1047,7 @@ int small_launch_with_scratch(const dqb_dense_problem* p, const dqb_ode_options*
   DenseSmallArgs a = make_args(p, o, out);
   a.counter = counter;
   a.slots = (float2*)slots;
+  if (int rc = solve_banded(a, counter, 0, 0, s)) return rc;
   const size_t smem = smem_for(NP, p->n_jumps);
   switch (NP) {
     case 16: mesolve_small_kernel<16><<<grid, kSmallThreads, smem, s>>>(a); break;
@@ -1041,7 +1067,7 @@ namespace dqb {
 template <int NP>
 __global__ void __launch_bounds__(kSmallThreads, NP == 64 ? 1 : (NP == 32 ? 3 : 4)) mesolve_ragged_kernel(const dqb_ragged_instance* __restrict__ d,
                                                                        long long count, CtrlOpts o, float2* slots,
-                                                                       unsigned int* counter) {
+                                                                       unsigned int* counter, const int* pend) {
   extern __shared__ float4 smem_raw[];
   __shared__ double red[40];
   __shared__ Ctrl ctl;
@@ -1055,31 +1081,11 @@ __global__ void __launch_bounds__(kSmallThreads, NP == 64 ? 1 : (NP == 32 ? 3 : 
     __syncthreads();
     const long long inst = ctl.inst;
     if (inst >= count) break;
-    const dqb_ragged_instance& r = d[inst];
-    InstView v;
-    v.n = r.n;
-    v.K = r.n_jumps;
-    v.nE = r.n_exp;
-    v.ntsave = r.n_tsave;
-    v.is_ket = r.rho0_is_ket;
-    v.save_states = r.save_states;
-    v.t0 = r.t0;
-    v.H = (const float2*)r.H;
-    v.L = (const float2*)r.L;
-    v.rho0 = (const float2*)r.rho0;
-    v.E = (const float2*)r.E;
-    v.tsave = r.tsave;
-    v.states = (float2*)r.states;
-    v.expects = (float2*)r.expects;
-    v.infos = r.infos;
-    v.status = r.status;
-    v.cancel = r.cancel;
-    v.inst = inst;
-    v.n_jump = 0;
-    v.jump_ts = nullptr;
-    v.tape_t = v.tape_h = nullptr;
-    v.tape_y = nullptr;
-    v.tape_cap = 0;
+    if (pend && pend[inst] != band::kPending) {  // the banded kernel has solved it
+      __syncthreads();  // every thread has read ctl.inst
+      continue;
+    }
+    const InstView v = view_of_ragged(d[inst], inst);
     SimtEngine<NP, 0> eng{sH, sX, sT, sL, v.n, v.K, o.form, nullptr, nullptr, inst};
     solve_one<NP>(eng, v, o, slot, red, ctl);
     __syncthreads();
@@ -1107,12 +1113,15 @@ static int ragged_grid_for(int NP, int K, long long count) {
 
 }  // namespace dqb
 
+static size_t ragged_marks_bytes(long long count) { return ((size_t)count * sizeof(int) + 255) & ~(size_t)255; }
+
 extern "C" size_t dqb_mesolve_ragged_workspace_size(int32_t max_n, int32_t max_jumps, int64_t count) {
   const int NP = pick_np(max_n);
   if (NP == 0 || count <= 0 || max_jumps < 0) return 0;
   const int g = ragged_grid_for(NP, max_jumps, count);
   if (g <= 0) return 0;
-  return 256 + (size_t)g * kSlotMats * NP * NP * sizeof(float2);
+  // work counters, one mark per instance (dqb_small_band.cuh), slots
+  return 256 + ragged_marks_bytes(count) + (size_t)g * kSlotMats * NP * NP * sizeof(float2);
 }
 
 extern "C" int dqb_mesolve_ragged(const dqb_ragged_instance* instances, int64_t count, int32_t max_n,
@@ -1134,13 +1143,27 @@ extern "C" int dqb_mesolve_ragged(const dqb_ragged_instance* instances, int64_t 
   cudaStream_t s = (cudaStream_t)stream;
   zero_words_kernel<<<1, 64, 0, s>>>((unsigned int*)workspace, 64);
   unsigned int* counter = (unsigned int*)workspace;
-  float2* slots = (float2*)((char*)workspace + 256);
+  int* marks = (int*)((char*)workspace + 256);
+  float2* slots = (float2*)((char*)workspace + 256 + ragged_marks_bytes(count));
   const CtrlOpts c = make_ctrl(*o);
+  const int* pend = nullptr;
+  if (c.form == DQB_FORM_HERMITIAN) {
+    band::Args b;
+    std::memset(&b, 0, sizeof(b));
+    b.d.batch = count;
+    b.d.o = c;
+    b.rag = instances;
+    b.counter = counter + 1;
+    b.pend = marks;
+    b.pend_stride = 1;
+    if (int rc = band::run(b, max_n, 0, s)) return rc;
+    pend = marks;
+  }
   const size_t smem = smem_for(NP, max_jumps);
   switch (NP) {
-    case 16: mesolve_ragged_kernel<16><<<grid, kSmallThreads, smem, s>>>(instances, count, c, slots, counter); break;
-    case 32: mesolve_ragged_kernel<32><<<grid, kSmallThreads, smem, s>>>(instances, count, c, slots, counter); break;
-    default: mesolve_ragged_kernel<64><<<grid, kSmallThreads, smem, s>>>(instances, count, c, slots, counter); break;
+    case 16: mesolve_ragged_kernel<16><<<grid, kSmallThreads, smem, s>>>(instances, count, c, slots, counter, pend); break;
+    case 32: mesolve_ragged_kernel<32><<<grid, kSmallThreads, smem, s>>>(instances, count, c, slots, counter, pend); break;
+    default: mesolve_ragged_kernel<64><<<grid, kSmallThreads, smem, s>>>(instances, count, c, slots, counter, pend); break;
   }
   return cudaGetLastError() == cudaSuccess ? DQB_OK : DQB_ERR_CUDA;
 }

@@ -61,6 +61,8 @@ struct DenseSmallArgs {
   float2* slots;
   unsigned int* counter;
   const int* order;  // start order of the instances, or null (0, 1, 2, ...)
+  const int* pend;   // take only the instances b with pend[b * pend_stride] == band::kPending
+  int pend_stride;   //   (dqb_small_band.cuh), or null: every instance
   CtrlOpts o;
   TdArgs td;
   // gradient tape (or null): per instance, the start time, size and starting state of
@@ -135,6 +137,35 @@ __device__ __forceinline__ InstView view_of(const DenseSmallArgs& a, long long i
   v.expects = a.expects ? a.expects + inst * a.nE * a.ntsave : nullptr;
   v.infos = a.infos ? a.infos + inst * 3 : nullptr;
   v.status = a.status ? a.status + inst : nullptr;
+  return v;
+}
+
+// The same for a ragged launch's instance.
+__device__ __forceinline__ InstView view_of_ragged(const dqb_ragged_instance& r, long long inst) {
+  InstView v;
+  v.n = r.n;
+  v.K = r.n_jumps;
+  v.nE = r.n_exp;
+  v.ntsave = r.n_tsave;
+  v.is_ket = r.rho0_is_ket;
+  v.save_states = r.save_states;
+  v.t0 = r.t0;
+  v.H = (const float2*)r.H;
+  v.L = (const float2*)r.L;
+  v.rho0 = (const float2*)r.rho0;
+  v.E = (const float2*)r.E;
+  v.tsave = r.tsave;
+  v.states = (float2*)r.states;
+  v.expects = (float2*)r.expects;
+  v.infos = r.infos;
+  v.status = r.status;
+  v.cancel = r.cancel;
+  v.inst = inst;
+  v.n_jump = 0;
+  v.jump_ts = nullptr;
+  v.tape_t = v.tape_h = nullptr;
+  v.tape_y = nullptr;
+  v.tape_cap = 0;
   return v;
 }
 

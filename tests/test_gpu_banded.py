@@ -1,0 +1,87 @@
+"""The banded kernel of the n <= 64 path (``csrc/dqb_dense_small_band.cu``) against the
+product kernel that solves every other instance: the same problem with 1e-25 added to every
+entry of H has full matrices, so it takes the product kernel, and differs by nothing that
+FP32 sums of these sizes can show.  Both sum the same products in the same order, so step
+counts are equal and states agree to the rounding of the dense-output weights."""
+
+import numpy as np
+import pytest
+import torch
+
+import dynamiqs_b200 as dq
+
+pytestmark = pytest.mark.gpu
+
+# every tile count of both thread layouts, at its edges
+SIZES = (1, 2, 7, 8, 9, 15, 16, 17, 24, 25, 31, 32, 33, 48, 49, 63, 64)
+
+
+def _band(rng, n, offsets, scale=1.0, hermitian=False):
+    m = np.zeros((n, n), complex)
+    for k in offsets:
+        if abs(k) < n:
+            v = scale * (rng.normal(size=n - abs(k)) + 1j * rng.normal(size=n - abs(k)))
+            m += np.diag(v, k)
+    return (m + m.conj().T) / 2 if hermitian else m
+
+
+def _problem(n, seed, batch, jumps):
+    rng = np.random.default_rng(seed)
+    H = np.stack([_band(rng, n, (0, 1, 3), 1.0, True) for _ in range(batch)])
+    Ls = [_band(rng, n, off, 0.3) for off in jumps]
+    E = _band(rng, n, range(-n + 1, n), 1.0, True) / max(n, 1)
+    g = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
+    rho = (g @ g.conj().T) / np.trace(g @ g.conj().T).real
+    c = lambda x: np.ascontiguousarray(x, dtype=np.complex64)  # noqa: E731
+    return c(H), [c(L) for L in Ls], c(rho), [c(E)]
+
+
+def _agree(a, b):
+    assert torch.equal(a.infos.nsteps, b.infos.nsteps)
+    assert torch.equal(a.infos.naccepted, b.infos.naccepted)
+    scale = b.states.abs().amax()
+    # unit trace, at most ~50 steps: eight roundings of the largest entry
+    assert (a.states - b.states).abs().amax() <= 8 * 2 ** -24 * max(float(scale), 1e-3) + 1e-9
+    assert (a.expects - b.expects).abs().amax() <= 1e-6
+
+
+@pytest.mark.parametrize('n, batch', [(n, 2) for n in SIZES] + [(n, 400) for n in SIZES if n <= 32])
+def test_same_as_product_kernel(cuda_device, n, batch):  # two thread layouts up to n = 32
+    H, Ls, rho, Es = _problem(n, n, batch, [(1,), (0,)])
+    ts = np.linspace(0.0, 0.5, 4)
+    got = dq.mesolve(H, Ls, rho, ts, exp_ops=Es, method=dq.Tsit5(rtol=1e-5, atol=1e-6))
+    ref = dq.mesolve(H + np.complex64(1e-25), Ls, rho, ts, exp_ops=Es, method=dq.Tsit5(rtol=1e-5, atol=1e-6))
+    _agree(got, ref)
+
+
+@pytest.mark.parametrize('jumps', [[], [(1, -1)], [(-2,), (0, 2)], [(-1,), (1,), (2,)]])
+@pytest.mark.parametrize('n', [13, 40])
+def test_jump_patterns_and_options(cuda_device, n, jumps):
+    H, Ls, rho, Es = _problem(n, 3, 3, jumps)
+    for kw in (dict(), dict(options=dq.Options(save_states=False)), dict(method=dq.Dopri5())):
+        got = dq.mesolve(H, Ls, rho, [0.1, 0.1, 0.4], exp_ops=Es, **kw)
+        ref = dq.mesolve(H + np.complex64(1e-25), Ls, rho, [0.1, 0.1, 0.4], exp_ops=Es, **kw)
+        _agree(got, ref)
+
+
+def test_mixed_batch_and_fallbacks(cuda_device):
+    """Full and banded instances of one batch each give what they give alone; a rho0 whose
+    triangles differ beyond rounding (within the hermiticity check) keeps the product
+    kernel's result; a rho0 that fails the check is refused."""
+    H, Ls, rho, Es = _problem(20, 5, 4, [(1,)])
+    H[1] += np.complex64(1e-25)
+    H[2] += _problem(20, 6, 1, [])[0][0].T * np.complex64(1e-25)
+    ts = [0.0, 0.3]
+    all_ = dq.mesolve(H, Ls, rho, ts, exp_ops=Es)
+    for b in range(4):
+        one = dq.mesolve(H[b], Ls, rho, ts, exp_ops=Es)
+        assert torch.equal(one.states, all_.states[b]) and int(one.infos.nsteps) == int(all_.infos.nsteps[b])
+    skew = rho.copy()
+    skew[2, 7] += np.complex64(5e-6)
+    a = dq.mesolve(H[0], Ls, skew, ts, exp_ops=Es)
+    b = dq.mesolve(H[1], Ls, skew, ts, exp_ops=Es)
+    assert torch.equal(a.infos.nsteps, dq.mesolve(H[0], Ls, skew, ts).infos.nsteps)
+    assert b.states.shape == a.states.shape and float((a.states[0] - torch.as_tensor(skew).cuda()).abs().max()) == 0.0
+    skew[2, 7] += np.complex64(1e-3)
+    with pytest.raises(RuntimeError, match='not hermitian'):
+        dq.mesolve(H[0], Ls, skew, ts)
