@@ -35,6 +35,8 @@ struct Term {
   float alpha;
 };
 
+#include "dqb_large_band.cuh"
+
 struct LargeOps {
   int n, K;
   const float2* H;  // [*, n, n]
@@ -46,6 +48,7 @@ struct LargeOps {
   float2* tmp;  // [B, n, n]
   const dqb_ragged_instance* rag;  // per-instance operators (ragged batches), or null
   int prec;                        // DQB_PREC_*: FP32 CUDA cores or a tensor-core mode
+  BandTabs band;                   // instances with banded operators (rec null: none)
 };
 
 __device__ __forceinline__ int jumps_of(const LargeOps& d, int b) { return d.rag ? d.rag[b].n_jumps : d.K; }
@@ -71,6 +74,9 @@ __device__ __forceinline__ bool job_skips(const big::Common& c, int b, int need_
   if (need_run == 1 ? !I.run : I.status != DQB_INST_OK) return true;
   return kry > 0 && I.kvalid >= kry + 2;
 }
+
+// Whether instance b's right-hand sides come from the stencil (dqb_large_band.cuh).
+__device__ __forceinline__ bool banded(const LargeOps& d, int b) { return d.band.rec && d.band.rec[b].ok; }
 
 constexpr int BM = 64, BN = 64, BK = 16, NT = 256;
 
@@ -151,7 +157,7 @@ __global__ void __launch_bounds__(NT) cgemm_kernel(big::Common c, LargeOps d, Ge
   const int Kz = job.kdst < 0 ? d.K : 1;
   const int b = blockIdx.z / Kz;
   const int kz = job.kdst < 0 ? (int)(blockIdx.z % Kz) : job.kdst;
-  if (job_skips(c, b, job.need_run, job.kry)) return;
+  if (job_skips(c, b, job.need_run, job.kry) || banded(d, b)) return;
   const int Kb = jumps_of(d, b);
   if (job.kdst < 0 && kz >= Kb) return;  // this instance has fewer jumps
   const int tiles = (n + BM - 1) / BM;
@@ -275,7 +281,7 @@ __global__ void __launch_bounds__(256) symmetrize_kernel(big::Common c, LargeOps
   if (ext_out) {
     out = ext_out + (long long)b * d.n * d.n;
   } else {
-    if (job_skips(c, b, need_run, kry)) return;
+    if (job_skips(c, b, need_run, kry) || banded(d, b)) return;
     const big::Inst& I = c.inst[b];
     out = big::slot(c, b, I.sk[out_k]);
     if (kry > 0) scale = (float)(kry == 1 ? I.tau * I.sig1 : I.tau);
@@ -313,6 +319,341 @@ __global__ void __launch_bounds__(256) symmetrize_kernel(big::Common c, LargeOps
     float2 v = tmp[(long long)gr * n + gc];
     out[(long long)gr * n + gc] = make_float2(v.x * scale, v.y * scale);
   }
+}
+
+// ------------------------------------------------------------------------------------
+// banded instances (dqb_large_band.cuh)
+// ------------------------------------------------------------------------------------
+
+__device__ __forceinline__ bool band_inactive(const big::Common& c, int b) {
+  return c.inst[b].status == big::kInactive;
+}
+
+// grid (tiles, 1 + K, B): the nonzero diagonals of H (blockIdx.y = 0) and of each jump.
+__global__ void __launch_bounds__(256) band_scan_kernel(big::Common c, LargeOps d) {
+  extern __shared__ unsigned band_bits[];
+  const int b = blockIdx.z, op = blockIdx.y, n = d.n, W = d.band.words;
+  if (band_inactive(c, b) || op - 1 >= jumps_of(d, b)) return;
+  for (int w = threadIdx.x; w < W; w += blockDim.x) band_bits[w] = 0u;
+  __syncthreads();
+  const float2* M = op == 0 ? src_ptr(c, d, b, SRC_H, 0, 0, nullptr) : src_ptr(c, d, b, SRC_L, op - 1, 0, nullptr);
+  for (int i = blockIdx.x; i < n; i += gridDim.x)
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+      const float2 v = M[(long long)i * n + j];
+      if (v.x != 0.f || v.y != 0.f) {
+        const int e = j - i + n - 1;
+        const unsigned bit = 1u << (e & 31);
+        if (!(*(volatile unsigned*)&band_bits[e >> 5] & bit)) atomicOr(&band_bits[e >> 5], bit);
+      }
+    }
+  __syncthreads();
+  unsigned* out = d.band.mask + ((long long)b * (1 + d.K) + op) * W;
+  for (int w = threadIdx.x; w < W; w += blockDim.x)
+    if (band_bits[w]) atomicOr(&out[w], band_bits[w]);
+}
+
+// One warp per instance: the list of diagonals, or ok = 0 when there are too many.
+__global__ void __launch_bounds__(32) band_lists_kernel(big::Common c, LargeOps d) {
+  __shared__ BandRec R;
+  const int b = blockIdx.x, lane = threadIdx.x, n = d.n, W = d.band.words;
+  const int K = band_inactive(c, b) ? 0 : jumps_of(d, b);
+  const unsigned* mask = d.band.mask + (long long)b * (1 + d.K) * W;
+  // offsets of the set bits of `m`, appended to list[count...max); false when they do not fit
+  auto append = [&](const unsigned* m, int* list, int max, int& count) {
+    for (int w0 = 0; w0 < W; w0 += 32) {
+      const unsigned mine = w0 + lane < W ? m[w0 + lane] : 0u;
+      unsigned busy = __ballot_sync(0xffffffffu, mine != 0u);
+      for (; busy; busy &= busy - 1) {
+        const int src = __ffs((int)busy) - 1;
+        for (unsigned x = __shfl_sync(0xffffffffu, mine, src); x; x &= x - 1) {
+          if (count == max) return false;
+          if (lane == 0) list[count] = 32 * (w0 + src) + __ffs((int)x) - 1 - (n - 1);
+          ++count;
+        }
+      }
+    }
+    return true;
+  };
+  bool ok = K <= kBandMaxK;
+  int nl = 0, nh = 0;
+  if (band_inactive(c, b)) {  // unused capacity: no work on either path
+    if (lane == 0) d.band.rec[b].ok = 1;
+    return;
+  }
+  for (int k = 0; ok && k < K; ++k) {
+    if (lane == 0) R.lstart[k] = nl;
+    ok = append(mask + (1 + k) * (long long)W, R.loff, kBandMaxL, nl);
+  }
+  ok = ok && append(mask, R.hoff, kBandMaxH, nh);
+  __syncwarp();
+  if (lane == 0) {
+    if (ok) {
+      R.lstart[K] = nl;
+      // the diagonals of L^+L join those of H, in ascending order
+      for (int k = 0; ok && k < K; ++k)
+        for (int p = R.lstart[k]; ok && p < R.lstart[k + 1]; ++p)
+          for (int q = R.lstart[k]; q < R.lstart[k + 1]; ++q) {
+            const int off = R.loff[q] - R.loff[p];
+            if (off <= -n || off >= n) continue;
+            int at = 0;
+            while (at < nh && R.hoff[at] < off) ++at;
+            if (at < nh && R.hoff[at] == off) continue;
+            if (nh == kBandMaxH) {
+              ok = false;
+              break;
+            }
+            for (int e = nh; e > at; --e) R.hoff[e] = R.hoff[e - 1];
+            R.hoff[at] = off;
+            ++nh;
+          }
+      R.nh = nh;
+      R.nk = K;
+    }
+    R.ok = ok;
+    atomicOr(d.band.work, ok ? 2 : 1);  // Work bits
+    d.band.rec[b] = R;
+  }
+}
+
+// Runs the one loop of three that the instances need (the index is their Work bits).
+__global__ void choose_loop_kernel(const int* work, LoopHandles h) {
+  for (int i = 0; i < LoopHandles::kCount; ++i) cudaGraphSetConditional(h.h[i], *work == i + 1 ? 1u : 0u);
+}
+
+// grid (ceil(n / 256), B): the diagonals of the jumps and of Hnh = -iH - 1/2 sum L^+L, with
+// the roundings of launch_hnh (a product's sum by ascending inner index, four jumps per
+// group, H added to the first group).
+__global__ void __launch_bounds__(256) band_tables_kernel(big::Common c, LargeOps d) {
+  const int b = blockIdx.y, n = d.n, i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (band_inactive(c, b) || i >= n) return;
+  const BandRec& R = d.band.rec[b];
+  if (!R.ok) return;
+  const long long nn = (long long)n * n;
+  const float2* H = src_ptr(c, d, b, SRC_H, 0, 0, nullptr);
+  const float2* L = R.nk > 0 ? src_ptr(c, d, b, SRC_L, 0, 0, nullptr) : nullptr;
+  for (int k = 0; k < R.nk; ++k)
+    for (int p = R.lstart[k]; p < R.lstart[k + 1]; ++p) {
+      const int j = i + R.loff[p];
+      d.band.ld[((long long)b * kBandMaxL + p) * n + i] =
+          j >= 0 && j < n ? L[k * nn + (long long)i * n + j] : make_float2(0.f, 0.f);
+    }
+  for (int q = 0; q < R.nh; ++q) {
+    const int j = i + R.hoff[q];
+    float2 v = make_float2(0.f, 0.f);
+    if (j >= 0 && j < n) {
+      int k = 0;
+      do {
+        float2 g = make_float2(0.f, 0.f);
+        for (int e = 0; e < 4 && k < R.nk; ++e, ++k) {
+          float2 s = make_float2(0.f, 0.f);
+          for (int p = R.lstart[k + 1] - 1; p >= R.lstart[k]; --p) {  // m = i - off ascends
+            const int m = i - R.loff[p];
+            if (m < 0 || m >= n) continue;
+            for (int t = R.lstart[k]; t < R.lstart[k + 1]; ++t)
+              if (m + R.loff[t] == j)
+                cmac(s, cconj(L[k * nn + (long long)m * n + i]), L[k * nn + (long long)m * n + j]);
+          }
+          g = caxpy(-0.5f, s, g);
+        }
+        if (k <= 4) {  // the first group
+          const float2 h = H[(long long)i * n + j];
+          v = make_float2(g.x + h.y, g.y - h.x);
+        } else {
+          v = cadd(g, v);
+        }
+      } while (k < R.nk);
+    }
+    d.band.hd[((long long)b * kBandMaxH + q) * n + i] = v;
+  }
+}
+
+// out = scale f(X) of a banded instance on the block's 32 x 32 tile: an upper tile of the
+// hermitian form, mirrored when `mirror`, or any tile of the standard form.  A thread has
+// four elements (big::HTile: NR rows of NC adjacent columns); in the hermitian form A =
+// tmp[i][j] and Bc = conj(tmp[j][i]).
+template <bool VEC>
+__device__ __forceinline__ void band_stencil(const LargeOps& d, int b, const float2* __restrict__ X,
+                                             float2* __restrict__ out, int herm, float scale, int mirror,
+                                             BandRec& R, float2 (*sh)[33]) {
+  constexpr int NR = VEC ? 2 : 4, NC = VEC ? 2 : 1;
+  for (int e = threadIdx.x; e < (int)(sizeof(BandRec) / sizeof(int)); e += blockDim.x)
+    reinterpret_cast<int*>(&R)[e] = reinterpret_cast<const int*>(d.band.rec + b)[e];
+  __syncthreads();
+  const int n = d.n, T = (n + 31) / 32;
+  int ti, tj;
+  if (herm) big::herm_tile(blockIdx.x, T, ti, tj);
+  else ti = blockIdx.x / T, tj = blockIdx.x % T;
+  const float2* __restrict__ hd = d.band.hd + (long long)b * kBandMaxH * n;
+  const float2* __restrict__ ld = d.band.ld + (long long)b * kBandMaxL * n;
+  const big::HTile<VEC> t;
+  // (an element outside the matrix repeats one inside; it is not stored.  n^2 < 2^31: the
+  // dense operators of a larger n would not fit the card)
+  int row[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) row[r] = min(ti * 32 + t.row(r * NC), n - 1);
+  const int col = min(tj * 32 + t.col(0), n - NC);
+  // X[i][s .. s + NC - 1]; beyond the matrix any entry will do, its coefficient is zero
+  auto read = [&](int i, int s, float2 (&x)[NC]) {
+    const float2* p = X + min(max(i, 0), n - 1) * n;
+    if (VEC && (s & 1) == 0 && s >= 0 && s < n) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(p + s));
+      x[0] = make_float2(v.x, v.y), x[NC - 1] = make_float2(v.z, v.w);
+    } else {
+#pragma unroll
+      for (int q = 0; q < NC; ++q) x[q] = __ldg(p + min(max(s + q, 0), n - 1));
+    }
+  };
+  float2 A[NR][NC], Bc[NR][NC];
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+#pragma unroll
+    for (int q = 0; q < NC; ++q) A[r][q] = Bc[r][q] = make_float2(0.f, 0.f);
+  for (int m = 0; m < R.nh; ++m) {
+    const int off = R.hoff[m];
+    float2 hc[NC];
+#pragma unroll
+    for (int q = 0; q < NC; ++q) hc[q] = cconj(__ldg(hd + m * n + col + q));
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      const float2 hr = __ldg(hd + m * n + row[r]);
+      float2 x[NC], y[NC];
+      read(row[r] + off, col, x);
+      if (off != 0) {
+        read(row[r], col + off, y);
+      } else {
+#pragma unroll
+        for (int q = 0; q < NC; ++q) y[q] = x[q];
+      }
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        A[r][q] = cfma(hr, x[q], A[r][q]);
+        Bc[r][q] = herm ? cfma(hc[q], y[q], Bc[r][q]) : cfma(y[q], hc[q], Bc[r][q]);
+      }
+    }
+  }
+  if (!herm) {
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+      for (int q = 0; q < NC; ++q) A[r][q] = cadd(A[r][q], Bc[r][q]);
+  }
+  const float half = herm ? 0.5f : 1.0f;
+  int k = 0;
+  for (int group = herm ? 3 : 2; k < R.nk; group = 4) {  // jumps per launch of launch_rhs
+    float2 ga[NR][NC], gb[NR][NC];
+    const bool first = k == 0;
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        ga[r][q] = first ? A[r][q] : make_float2(0.f, 0.f);
+        gb[r][q] = first ? Bc[r][q] : make_float2(0.f, 0.f);
+      }
+    for (int g = 0; g < group && k < R.nk; ++g, ++k) {
+      const int p0 = R.lstart[k], p1 = R.lstart[k + 1];
+      if (p1 == p0 + 1) {  // one diagonal: the same X for both sums
+        const int off = R.loff[p0];
+        const float2 z = make_float2(0.f, 0.f);
+        float2 lc[NC];
+#pragma unroll
+        for (int q = 0; q < NC; ++q) lc[q] = cconj(__ldg(ld + p0 * n + col + q));
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+          const float2 lr = __ldg(ld + p0 * n + row[r]);
+          float2 x[NC];
+          read(row[r] + off, col + off, x);
+#pragma unroll
+          for (int q = 0; q < NC; ++q) {
+            const float2 u = cfma(lr, x[q], z), w = cfma(lc[q], x[q], z);
+            ga[r][q] = cadd(ga[r][q], cfma(make_float2(half * u.x, half * u.y), lc[q], z));
+            if (herm) gb[r][q] = cadd(gb[r][q], cfma(make_float2(half * w.x, half * w.y), lr, z));
+          }
+        }
+        continue;
+      }
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        float2 sa[NC], sb[NC], u[NC], x[NC];
+#pragma unroll
+        for (int q = 0; q < NC; ++q) sa[q] = sb[q] = make_float2(0.f, 0.f);
+        for (int m = p0; m < p1; ++m) {  // (L X / 2)[i][j + m] conj(L[j][j + m])
+#pragma unroll
+          for (int q = 0; q < NC; ++q) u[q] = make_float2(0.f, 0.f);
+          for (int p = p0; p < p1; ++p) {
+            const float2 lr = __ldg(ld + p * n + row[r]);
+            read(row[r] + R.loff[p], col + R.loff[m], x);
+#pragma unroll
+            for (int q = 0; q < NC; ++q) u[q] = cfma(lr, x[q], u[q]);
+          }
+#pragma unroll
+          for (int q = 0; q < NC; ++q)
+            sa[q] = cfma(make_float2(half * u[q].x, half * u[q].y), cconj(__ldg(ld + m * n + col + q)), sa[q]);
+        }
+        for (int p = p0; herm && p < p1; ++p) {  // the conjugate of the same at (j, i)
+#pragma unroll
+          for (int q = 0; q < NC; ++q) u[q] = make_float2(0.f, 0.f);
+          for (int m = p0; m < p1; ++m) {
+            read(row[r] + R.loff[p], col + R.loff[m], x);
+#pragma unroll
+            for (int q = 0; q < NC; ++q) u[q] = cfma(cconj(__ldg(ld + m * n + col + q)), x[q], u[q]);
+          }
+          const float2 lr = __ldg(ld + p * n + row[r]);
+#pragma unroll
+          for (int q = 0; q < NC; ++q) sb[q] = cfma(make_float2(half * u[q].x, half * u[q].y), lr, sb[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < NC; ++q) {
+          ga[r][q] = cadd(ga[r][q], sa[q]);
+          gb[r][q] = cadd(gb[r][q], sb[q]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        A[r][q] = first ? ga[r][q] : cadd(ga[r][q], A[r][q]);
+        Bc[r][q] = first ? gb[r][q] : cadd(gb[r][q], Bc[r][q]);
+      }
+  }
+  float2 v[4];
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      const float2 x = herm ? cadd(A[r][q], Bc[r][q]) : A[r][q];
+      v[r * NC + q] = make_float2(x.x * scale, x.y * scale);
+    }
+  if (herm && mirror) {
+    big::herm_store<VEC>(out, n, ti, tj, v, sh);
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    if (!big::htile_in<VEC>(n, ti, tj, r * NC)) continue;
+    float2* o = out + (long long)row[r] * n + col;
+    if (VEC) {
+      *reinterpret_cast<float4*>(o) = make_float4(v[2 * r].x, v[2 * r].y, v[2 * r + 1].x, v[2 * r + 1].y);
+    } else {
+      *o = v[r];
+    }
+  }
+}
+
+// k = f(X) of the banded instances.  grid (T (T + 1) / 2, B) in the hermitian form, (T * T, B)
+// in the standard one.  kry = q > 0: a Krylov basis right-hand side, times tau (and sig1 for
+// q = 1).  `mirror`: the hermitian form writes the lower triangle too.
+template <bool VEC>
+__global__ void __launch_bounds__(256) band_rhs_kernel(big::Common c, LargeOps d, int in_sel, int out_k,
+                                                       int need_run, int herm, int kry, int mirror) {
+  __shared__ float2 sh[32][33];
+  __shared__ BandRec R;
+  const int b = blockIdx.y;
+  if (job_skips(c, b, need_run, kry) || !d.band.rec[b].ok) return;
+  const big::Inst& I = c.inst[b];
+  const float scale = kry > 0 ? (float)(kry == 1 ? I.tau * I.sig1 : I.tau) : 1.f;
+  band_stencil<VEC>(d, b, src_ptr(c, d, b, SRC_IN, 0, in_sel, nullptr), big::slot(c, b, I.sk[out_k]), herm, scale,
+                    mirror, R, sh);
 }
 
 // ------------------------------------------------------------------------------------
@@ -496,7 +837,7 @@ __global__ void __launch_bounds__(tcg::kThreads, 1)
   const int Kz = job.kdst < 0 ? d.K : 1;
   const int b = blockIdx.z / Kz;
   const int kz = job.kdst < 0 ? (int)(blockIdx.z % Kz) : job.kdst;
-  if (job_skips(c, b, job.need_run, job.kry)) return;
+  if (job_skips(c, b, job.need_run, job.kry) || banded(d, b)) return;
   const int Kb = jumps_of(d, b);
   if (job.kdst < 0 && kz >= Kb) return;
   const int tiles = (n + 127) >> 7;
@@ -733,7 +1074,9 @@ void launch_gemm(cudaStream_t s, const big::Common& c, const LargeOps& d, const 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct LargeLayout {
-  size_t off_iter, off_inst, off_eacc, off_hnh, off_T, off_tmp, off_mats, total;
+  size_t off_iter, off_inst, off_eacc, off_hnh, off_T, off_tmp, off_mats, off_band, total;
+  size_t band_mask, band_hd, band_ld;  // from off_band
+  int band_words;
 };
 
 LargeLayout large_layout(int n, int K, int nE, int ntsave, long long B) {
@@ -746,14 +1089,37 @@ LargeLayout large_layout(int n, int K, int nE, int ntsave, long long B) {
   l.off_T = align_up(l.off_hnh + B * nn * sizeof(float2));
   l.off_tmp = align_up(l.off_T + B * (size_t)K * nn * sizeof(float2));
   l.off_mats = align_up(l.off_tmp + B * nn * sizeof(float2));
-  l.total = l.off_mats + B * (size_t)big::kSlots * nn * sizeof(float2);
+  l.off_band = align_up(l.off_mats + B * (size_t)big::kSlots * nn * sizeof(float2));
+  l.band_words = (2 * n - 1 + 31) / 32;
+  l.band_mask = align_up(B * sizeof(BandRec));
+  l.band_hd = align_up(l.band_mask + B * (size_t)(1 + K) * l.band_words * sizeof(unsigned));
+  l.band_ld = l.band_hd + B * (size_t)kBandMaxH * n * sizeof(float2);
+  l.total = l.off_band + l.band_ld + B * (size_t)kBandMaxL * n * sizeof(float2);
   return l;
 }
 
-// The three launches of one right-hand side (T_k, tmp, symmetrize).
+// What the instances of a loop need: the products (some instance has full operators), the
+// stencil (some instance is banded).
+enum Work : int { WORK_PRODUCTS = 1, WORK_STENCIL = 2 };
+
+// One right-hand side: the three launches of the products (T_k, tmp, symmetrize) and the
+// stencil of the banded instances, as far as `work` asks for them.
 void launch_rhs(cudaStream_t s, const big::Common& c, const LargeOps& d, int B, int in_sel, int out_k,
-                int need_run, int form, const float2* ext_in, float2* ext_out, int kry = 0) {
+                int need_run, int form, const float2* ext_in, float2* ext_out, int kry = 0,
+                int work = WORK_PRODUCTS | WORK_STENCIL) {
   const int n = d.n;
+  const bool herm = form == DQB_FORM_HERMITIAN;
+  const int t32 = (n + 31) / 32;
+  const dim3 g32 = herm ? big::herm_grid(n, B) : dim3(t32 * t32, B);
+  if (d.band.rec && (work & WORK_STENCIL)) {
+    // a stage slot inside the loop is read by the hermitian-half kernels alone
+    const int mirror = need_run == 0 || kry > 0;
+    if (big::herm_vec(c))
+      band_rhs_kernel<true><<<g32, 256, 0, s>>>(c, d, in_sel, out_k, need_run, herm, kry, mirror);
+    else
+      band_rhs_kernel<false><<<g32, 256, 0, s>>>(c, d, in_sel, out_k, need_run, herm, kry, mirror);
+  }
+  if (!(work & WORK_PRODUCTS)) return;
   const bool tcp = use_tc(d, form);
   const float sc = form == DQB_FORM_HERMITIAN ? 0.5f : 1.0f;
   if (d.K > 0) {
@@ -789,10 +1155,7 @@ void launch_rhs(cudaStream_t s, const big::Common& c, const LargeOps& d, int B, 
     j2.accumulate = 1;
     nt = 0;
   }
-  const int t32 = (n + 31) / 32;
-  const bool herm = form == DQB_FORM_HERMITIAN;
-  symmetrize_kernel<<<herm ? big::herm_grid(n, B) : dim3(t32 * t32, B), 256, 0, s>>>(c, d, out_k, need_run, herm, kry,
-                                                       ext_out);
+  symmetrize_kernel<<<g32, 256, 0, s>>>(c, d, out_k, need_run, herm, kry, ext_out);
 }
 
 int check_dense_large(const dqb_dense_problem* p) {
@@ -892,6 +1255,28 @@ LargeOps make_ops(const dqb_dense_problem* p, char* ws, const LargeLayout& lay) 
   return d;
 }
 
+// The tables of the banded instances (solves with constant operators).
+void use_band(LargeOps* d, char* ws, const LargeLayout& lay) {
+  char* base = ws + lay.off_band;
+  d->band.rec = (BandRec*)base;
+  d->band.mask = (unsigned*)(base + lay.band_mask);
+  d->band.words = lay.band_words;
+  d->band.hd = (float2*)(base + lay.band_hd);
+  d->band.ld = (float2*)(base + lay.band_ld);
+  d->band.work = (int*)(ws + lay.off_iter) + 4;
+}
+
+// Lists and tables of the banded instances (after setup_kernel).
+void launch_band_setup(cudaStream_t s, const big::Common& c, const LargeOps& d, int B) {
+  const size_t words = (size_t)B * (1 + d.K) * d.band.words;
+  zero_words_kernel<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(d.band.mask, (int)words);
+  zero_words_kernel<<<1, 32, 0, s>>>((unsigned*)d.band.work, 1);
+  band_scan_kernel<<<dim3(std::min(d.n, std::max(1, 1184 / B)), 1 + d.K, B), 256,
+                     d.band.words * sizeof(unsigned), s>>>(c, d);
+  band_lists_kernel<<<B, 32, 0, s>>>(c, d);
+  band_tables_kernel<<<dim3((d.n + 255) / 256, B), 256, 0, s>>>(c, d);
+}
+
 void launch_hnh(cudaStream_t s, const big::Common& c, const LargeOps& d, int B, int need_run) {
   const int tiles = (d.n + BM - 1) / BM;
   GemmJob j;
@@ -945,6 +1330,12 @@ static void init_carveouts() {
     prefer_max_shared(zero_words_kernel);
     prefer_max_shared(cgemm_kernel);
     prefer_max_shared(symmetrize_kernel);
+    prefer_max_shared(band_rhs_kernel<true>);
+    prefer_max_shared(band_rhs_kernel<false>);
+    prefer_max_shared(band_scan_kernel);
+    prefer_max_shared(band_lists_kernel);
+    prefer_max_shared(band_tables_kernel);
+    prefer_max_shared(choose_loop_kernel);
     prefer_max_shared(hnh_td_dense_kernel);
     prefer_max_shared(lt_td_dense_kernel);
     auto tc_attrs = [](auto kern, int smem) {
@@ -1005,6 +1396,7 @@ static int run_large(const big::Common& c, const LargeOps& d_in, cudaStream_t s,
 
   big::setup_kernel<<<gi, 128, 0, s>>>(c);
   big::load_rho0_kernel<<<ge, T, 0, s>>>(c);
+  if (d.band.rec) launch_band_setup(s, c, d, B);
   if (!jtv.on) {  // (with time-dependent jump operators every Hnh is formed at its time)
     LargeOps d0 = d;  // the constant Hnh: into hnh, or into hnh0 when H depends on time
     if (timedep) d0.hnh = hnh0;
@@ -1027,9 +1419,9 @@ static int run_large(const big::Common& c, const LargeOps& d_in, cudaStream_t s,
   big::init_ctrl_kernel<<<gi, 128, 0, s>>>(c, 1);
   if (cudaGetLastError() != cudaSuccess) return DQB_ERR_CUDA;
 
-  auto body = [&](cudaStream_t cs, cudaGraphConditionalHandle h, int* flag) {
+  auto iteration = [&](cudaStream_t cs, cudaGraphConditionalHandle h, int* flag, int work) {
     if (krylov) {
-      for (int q = 1; q <= 6; ++q) launch_rhs(cs, c, d, B, q + 2, q, 1, form, nullptr, nullptr, q);
+      for (int q = 1; q <= 6; ++q) launch_rhs(cs, c, d, B, q + 2, q, 1, form, nullptr, nullptr, q, work);
       big::launch_kry_combine(cs, c, ge);
       big::control_kernel<<<gi, 128, 0, cs>>>(c);
       big::launch_save(cs, c, ge, 2);
@@ -1040,11 +1432,11 @@ static int run_large(const big::Common& c, const LargeOps& d_in, cudaStream_t s,
     for (int st = 0; st < 5; ++st) {
       big::launch_combine(cs, c, ge, st);
       at_time(cs, st + 1);
-      launch_rhs(cs, c, d, B, 2, st + 1, 1, form, nullptr, nullptr);
+      launch_rhs(cs, c, d, B, 2, st + 1, 1, form, nullptr, nullptr, 0, work);
     }
     big::launch_combine(cs, c, ge, 5);
     at_time(cs, 6);
-    launch_rhs(cs, c, d, B, 1, 6, 1, form, nullptr, nullptr);
+    launch_rhs(cs, c, d, B, 1, 6, 1, form, nullptr, nullptr, 0, work);
     big::launch_error(cs, c, ge);
     big::control_kernel<<<gi, 128, 0, cs>>>(c);
     big::launch_save(cs, c, ge, 1);
@@ -1055,8 +1447,14 @@ static int run_large(const big::Common& c, const LargeOps& d_in, cudaStream_t s,
       launch_rhs(cs, c, d, B, 0, 0, 3, form, nullptr, nullptr);
     }
   };
+  auto body = [&](cudaStream_t cs, cudaGraphConditionalHandle h, int* flag) { iteration(cs, h, flag, WORK_PRODUCTS); };
   if (host_loop_requested()) {
-    if (run_host_loop(body, (int*)(c.iter + 1), s) != cudaSuccess) return DQB_ERR_CUDA;
+    int work = WORK_PRODUCTS;
+    if (d.band.rec && (cudaMemcpyAsync(&work, d.band.work, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+                       cudaStreamSynchronize(s) != cudaSuccess))
+      return DQB_ERR_CUDA;
+    auto chosen = [&](cudaStream_t cs, cudaGraphConditionalHandle h, int* flag) { iteration(cs, h, flag, work); };
+    if (run_host_loop(chosen, (int*)(c.iter + 1), s) != cudaSuccess) return DQB_ERR_CUDA;
   } else {
     LaunchKey key;
     std::memset(&key, 0, sizeof(key));
@@ -1070,7 +1468,17 @@ static int run_large(const big::Common& c, const LargeOps& d_in, cudaStream_t s,
     key.krylov = krylov;
     cudaGraphExec_t exec = g_cache.find(&key, sizeof(key));
     if (!exec) {
-      if (build_while_graph(body, &exec) != cudaSuccess) return DQB_ERR_CUDA;
+      const cudaError_t err =
+          d.band.rec ? build_choice_graph(
+                           [&](cudaStream_t cs, const LoopHandles& h) {
+                             choose_loop_kernel<<<1, 1, 0, cs>>>(d.band.work, h);
+                           },
+                           [&](cudaStream_t cs, cudaGraphConditionalHandle h, int loop) {
+                             iteration(cs, h, nullptr, loop + 1);
+                           },
+                           &exec)
+                     : build_while_graph(body, &exec);
+      if (err != cudaSuccess) return DQB_ERR_CUDA;
       g_cache.insert(&key, sizeof(key), exec, s);
     } else {
       g_cache.touch(&key, sizeof(key), s);
@@ -1149,6 +1557,7 @@ extern "C" int dqb_mesolve_dense_large_ragged(const dqb_ragged_instance* instanc
   LargeOps d = make_ops(&p, ws, lay);
   d.rag = instances;
   d.prec = o->precision;
+  use_band(&d, ws, lay);
   big::Common c;
   std::memset(&c, 0, sizeof(c));
   c.n = n;
@@ -1225,7 +1634,10 @@ static int solve_large(const dqb_dense_problem* p, const dqb_td_hamiltonian* tdh
   c.rho0 = (const float2*)p->rho0;
   c.ridx = p->rho0_index;
   c.iter = (long long*)(ws + lay.off_iter);
-  if (!tdh) return run_large(c, d, (cudaStream_t)stream, large_krylov(*o));
+  if (!tdh) {
+    use_band(&d, ws, lay);
+    return run_large(c, d, (cudaStream_t)stream, large_krylov(*o));
+  }
   c.n_jump = tdh->n_jump_ts;
   c.jump_ts = tdh->jump_ts;
   return run_large(c, d, (cudaStream_t)stream, false, &td, (float2*)(ws + align_up(lay.total)), &jt,

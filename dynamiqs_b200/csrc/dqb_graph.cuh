@@ -111,40 +111,87 @@ cudaError_t run_host_loop(Body body, int* flag, cudaStream_t s) {
   }
 }
 
-// Build "WHILE (cond) { body }" where `body(stream, handle, nullptr)` enqueues one loop
-// iteration on the capture stream and must end with a kernel that sets the condition.
+// Adds "WHILE (handle) { body }" to `g` after `dep` (or at its start): `body(stream, handle,
+// nullptr)` enqueues one loop iteration on the capture stream `cap` and must end with a
+// kernel that sets the condition.
+template <class Body>
+cudaError_t add_while_node(cudaGraph_t g, cudaGraphConditionalHandle handle, const cudaGraphNode_t* dep,
+                           cudaStream_t cap, Body body, cudaGraphNode_t* node) {
+  cudaGraphNodeParams p = {cudaGraphNodeTypeConditional};
+  p.type = cudaGraphNodeTypeConditional;
+  p.conditional.handle = handle;
+  p.conditional.type = cudaGraphCondTypeWhile;
+  p.conditional.size = 1;
+  cudaError_t err = cudaGraphAddNode(node, g, dep, dep ? 1 : 0, &p);
+  if (err != cudaSuccess) return err;
+  cudaGraph_t bodyg = p.conditional.phGraph_out[0];
+  err = cudaStreamBeginCaptureToGraph(cap, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+  if (err != cudaSuccess) return err;
+  body(cap, handle, (int*)nullptr);
+  err = cudaStreamEndCapture(cap, &bodyg);
+  return err == cudaSuccess ? cudaGetLastError() : err;
+}
+
+// Build "WHILE (cond) { body }" (add_while_node).
 template <class Body>
 cudaError_t build_while_graph(Body body, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   cudaError_t err = cudaGraphCreate(&g, 0);
   if (err != cudaSuccess) return err;
-  cudaGraphConditionalHandle handle;
-  err = cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault);
+  cudaStream_t cap = nullptr;
+  err = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
   if (err == cudaSuccess) {
-    cudaGraphNodeParams p = {cudaGraphNodeTypeConditional};
-    p.type = cudaGraphNodeTypeConditional;
-    p.conditional.handle = handle;
-    p.conditional.type = cudaGraphCondTypeWhile;
-    p.conditional.size = 1;
+    cudaGraphConditionalHandle handle;
     cudaGraphNode_t node;
-    err = cudaGraphAddNode(&node, g, nullptr, 0, &p);
-    if (err == cudaSuccess) {
-      cudaGraph_t bodyg = p.conditional.phGraph_out[0];
-      cudaStream_t cap;
-      err = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
-      if (err == cudaSuccess) {
-        err = cudaStreamBeginCaptureToGraph(cap, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-        if (err == cudaSuccess) {
-          body(cap, handle, (int*)nullptr);
-          cudaError_t e2 = cudaStreamEndCapture(cap, &bodyg);
-          if (err == cudaSuccess) err = e2;
-          if (err == cudaSuccess) err = cudaGetLastError();
-        }
-        cudaStreamDestroy(cap);
-      }
-      if (err == cudaSuccess) err = cudaGraphInstantiate(out, g, 0);
-    }
+    err = cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault);
+    if (err == cudaSuccess) err = add_while_node(g, handle, nullptr, cap, body, &node);
+    cudaStreamDestroy(cap);
   }
+  if (err == cudaSuccess) err = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  return err;
+}
+
+// Conditions of the loops of build_choice_graph.
+struct LoopHandles {
+  static constexpr int kCount = 3;
+  cudaGraphConditionalHandle h[kCount];
+};
+
+// Build "choose; WHILE (h[0]) { body(0) }; WHILE (h[1]) { body(1) }; ...": `choose(stream, handles)`
+// enqueues one kernel that sets the conditions (all 0 before it), so that the launch runs
+// one of the loops; `body(stream, handle, i)` enqueues an iteration of loop i.
+template <class Choose, class Body>
+cudaError_t build_choice_graph(Choose choose, Body body, cudaGraphExec_t* out) {
+  cudaGraph_t g = nullptr;
+  cudaError_t err = cudaGraphCreate(&g, 0);
+  if (err != cudaSuccess) return err;
+  cudaStream_t cap = nullptr;
+  err = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
+  if (err == cudaSuccess) {
+    LoopHandles hs;
+    cudaGraphNode_t node;
+    size_t count = 1;
+    for (int i = 0; i < LoopHandles::kCount && err == cudaSuccess; ++i)
+      err = cudaGraphConditionalHandleCreate(&hs.h[i], g, 0, cudaGraphCondAssignDefault);
+    if (err == cudaSuccess)
+      err = cudaStreamBeginCaptureToGraph(cap, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    if (err == cudaSuccess) {
+      choose(cap, hs);
+      err = cudaStreamEndCapture(cap, &g);
+      if (err == cudaSuccess) err = cudaGetLastError();
+    }
+    if (err == cudaSuccess) err = cudaGraphGetNodes(g, &node, &count);
+    if (err == cudaSuccess && count != 1) err = cudaErrorUnknown;
+    for (int i = 0; i < LoopHandles::kCount && err == cudaSuccess; ++i) {
+      const cudaGraphNode_t before = node;
+      err = add_while_node(
+          g, hs.h[i], &before, cap,
+          [&](cudaStream_t cs, cudaGraphConditionalHandle h, int*) { body(cs, h, i); }, &node);
+    }
+    cudaStreamDestroy(cap);
+  }
+  if (err == cudaSuccess) err = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
   return err;
 }

@@ -85,3 +85,36 @@ def test_mixed_batch_and_fallbacks(cuda_device):
     skew[2, 7] += np.complex64(1e-3)
     with pytest.raises(RuntimeError, match='not hermitian'):
         dq.mesolve(H[0], Ls, skew, ts)
+
+
+# ---- n > 64 in dense storage (csrc/dqb_large_band.cuh): the stencil against the products ----
+
+
+@pytest.mark.parametrize('n', [65, 66, 96, 97, 130])  # edges of the 32 x 32 tiles, odd rows
+@pytest.mark.parametrize('jumps', [[], [(1,)], [(0,), (-33,), (2, 5), (1,), (-1,)]])
+@pytest.mark.parametrize('form', ['hermitian', 'standard', 'krylov'])
+def test_large_same_as_products(cuda_device, n, jumps, form):
+    H, Ls, rho, Es = _problem(n, n + len(jumps), 2, jumps)
+    opts = dict(hermitian=dq.Options(), standard=dq.Options(assume_hermitian=False),
+                krylov=dq.Options(stepper='krylov'))[form]
+    ts = [0.0, 0.1, 0.25]
+    got = dq.mesolve(H, Ls, rho, ts, exp_ops=Es, options=opts)
+    ref = dq.mesolve(H + np.complex64(1e-25), Ls, rho, ts, exp_ops=Es, options=opts)
+    _agree(got, ref)
+
+
+def test_large_mixed_batch_and_tensor_cores(cuda_device):
+    """A batch of banded and full instances runs both kinds of kernels; each instance gives
+    what it gives alone (another loop of the graph), and with a tensor-core precision the
+    banded ones give the FP32 result."""
+    H, Ls, rho, Es = _problem(96, 8, 3, [(1,), (0,)])
+    full = H.copy()
+    full[1] += np.complex64(1e-25)
+    ts = [0.0, 0.2]
+    got = dq.mesolve(full, Ls, rho, ts, exp_ops=Es)
+    alone = [dq.mesolve(full[b], Ls, rho, ts, exp_ops=Es) for b in range(3)]
+    for b in range(3):
+        assert int(got.infos.nsteps[b]) == int(alone[b].infos.nsteps)
+        assert (got.states[b] - alone[b].states).abs().amax() <= 1e-7
+    tc = dq.mesolve(H, Ls, rho, ts, exp_ops=Es, options=dq.Options(precision='tf32x3'))
+    _agree(tc, dq.mesolve(H, Ls, rho, ts, exp_ops=Es))
