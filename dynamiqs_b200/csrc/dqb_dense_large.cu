@@ -8,11 +8,10 @@
 // Hnh = -iH - 1/2 sum L^+L is computed once per instance by the same GEMM.  The RK loop is
 // the stepper of dqb_big.cuh run as a CUDA-graph WHILE node.
 //
-// GEMM: 64 x 64 output tile per CTA, K-slices of 16 staged in shared memory (A stored
-// k-major so both operands are read as rows), 256 threads x (4 x 4) complex outputs,
-// FP32 FMA; each K-slice is read from global memory into registers (coalesced along the
-// operand's rows, transposed on the way into shared memory when the operand is a ^+).
-// Any n (edges zero-filled).
+// GEMM (cgemm_kernel): 32 to 80 square output tiles per CTA (cgemm_tile), K-slices of 16
+// copied asynchronously into a ring of three shared-memory stages (transposed on the way
+// when the operand is read across its rows), 256 threads x (2 x 2 to 5 x 5) complex outputs,
+// FP32 FMA.  Any n (edges zero-filled).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -78,8 +77,6 @@ __device__ __forceinline__ bool job_skips(const big::Common& c, int b, int need_
 // Whether instance b's right-hand sides come from the stencil (dqb_large_band.cuh).
 __device__ __forceinline__ bool banded(const LargeOps& d, int b) { return d.band.rec && d.band.rec[b].ok; }
 
-constexpr int BM = 64, BN = 64, BK = 16, NT = 256;
-
 __device__ __forceinline__ const float2* src_ptr(const big::Common& c, const LargeOps& d, int b, int src, int k,
                                                  int in_sel, const float2* ext_in) {
   const long long nn = (long long)d.n * d.n;
@@ -106,53 +103,95 @@ __device__ __forceinline__ const float2* src_ptr(const big::Common& c, const Lar
   }
 }
 
-// Load a BK x BM slice of op(M) (rows r0.., k-columns k0..) into S[k][m] (k-major).
-// op 0: op(M)[r][k] = M[r][k];  op 1: op(M)[r][k] = conj(M[k][r]).
-__device__ __forceinline__ void load_slice(float2 (&reg)[4], const float2* __restrict__ M, int n, int r0, int k0,
-                                           int op) {
-  const int tid = threadIdx.x;
+// One term of a job with the instance's own operands, in shared memory.
+struct TermPtrs {
+  const float2 *A, *B;
+  int opA, opB;
+  float alpha;
+};
+
+// FP32 product tile: 16 R x 16 R outputs per CTA, 256 threads with R x R each (rows ty + 16 i,
+// columns tx + 16 j), K-slices of 16 in a ring of three shared-memory stages, [k][row] and
+// [k][column] with an odd row stride (the transposing copies and the reads are both free of
+// bank conflicts).  Bound: issue slots and the operand ports (FMA is 64 of 72 instructions of a
+// step at R = 4; 62% of the cycles issue with one CTA per SM, 40 TFLOP/s of the 66 that
+// independent FMAs reach at n = 256 with many).
+constexpr int NT = 256, BK = 16, kRing = 3;
+
+template <int R>
+struct Tile {
+  static constexpr int T = 16 * R;
+  static constexpr int LD = T + 1;
+  static constexpr int kOperand = BK * LD;                                  // values of one slice
+  static constexpr int kSmem = kRing * 2 * kOperand * (int)sizeof(float2);  // bytes
+};
+
+// Asynchronous copy of one complex value into shared memory; zero when !in.
+__device__ __forceinline__ void copy_value(float2* dst, const float2* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(tc::smem_u32(dst)), "l"(src), "r"(in ? 8 : 0)
+               : "memory");
+}
+
+// The slice [k0, k0 + 16) of rows l0.. of M: S[k][l] = M[l0 + l][k0 + k], or, `across`, of
+// columns l0..: S[k][l] = M[k0 + k][l0 + l].  16 consecutive threads read 16 values of a row
+// of M: a thread's values lie 16 rows (columns) apart.
+template <int R>
+__device__ __forceinline__ void copy_slice(float2* S, const float2* __restrict__ M, int n, int l0, int k0, bool across) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int k = across ? ty : tx, l = across ? tx : ty;
+  const float2* src = M + (across ? (long long)(k0 + k) * n + l0 + l : (long long)(l0 + l) * n + k0 + k);
+  const long long step = across ? 16 : 16ll * n;
+  float2* dst = S + k * Tile<R>::LD + l;
+  const int rows = k0 + k < n ? n - l0 - l : 0;  // value q lies inside the matrix when 16 q < rows
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int e = tid + q * NT;  // 0..1023 over (BM x BK)
-    int r, k;
-    if (op == 0) {  // consecutive threads walk k (contiguous in M's rows)
-      r = e / BK;
-      k = e % BK;
-    } else {        // consecutive threads walk r (contiguous in M's rows k)
-      k = e / BM;
-      r = e % BM;
-    }
-    const int gr = r0 + r, gk = k0 + k;
-    float2 v = make_float2(0.f, 0.f);
-    if (gr < n && gk < n) {
-      v = op == 0 ? M[(long long)gr * n + gk] : cconj(M[(long long)gk * n + gr]);
-    }
-    reg[q] = v;
+  for (int q = 0; q < R; ++q) {
+    const bool in = 16 * q < rows;
+    copy_value(dst + 16 * q, in ? src + q * step : M, in);
   }
 }
 
-__device__ __forceinline__ void store_slice(float2* S, const float2 (&reg)[4], int op) {
-  const int tid = threadIdx.x;
+// acc += the slice's products, by ascending k; CA, CB: conjugated operands.
+template <int R, bool CA, bool CB>
+__device__ __forceinline__ void mac_slice(float2 (&acc)[R][R], const float2* __restrict__ As,
+                                          const float2* __restrict__ Bs) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll 4  // (all 16 steps: 28 KB of code at R = 5, and the warps wait for instructions)
+  for (int k = 0; k < BK; ++k) {
+    float2 a[R], b[R];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int e = tid + q * NT;
-    int r, k;
-    if (op == 0) {
-      r = e / BK;
-      k = e % BK;
-    } else {
-      k = e / BM;
-      r = e % BM;
+    for (int i = 0; i < R; ++i) {
+      a[i] = As[k * Tile<R>::LD + ty + 16 * i];
+      b[i] = Bs[k * Tile<R>::LD + tx + 16 * i];
+      if (CA) a[i].y = -a[i].y;
+      if (CB) b[i].y = -b[i].y;
     }
-    S[k * (BM + 1) + r] = reg[q];
+    // the two FMAs of a part that depend on each other are R * R instructions apart
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        acc[i][j].x = fmaf(a[i].x, b[j].x, acc[i][j].x);
+        acc[i][j].y = fmaf(a[i].x, b[j].y, acc[i][j].y);
+      }
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        acc[i][j].x = fmaf(-a[i].y, b[j].y, acc[i][j].x);
+        acc[i][j].y = fmaf(a[i].y, b[j].x, acc[i][j].y);
+      }
   }
 }
 
-// grid (tiles_n * tiles_n, 1, B * Kz): one 64 x 64 tile of C = sum_terms alpha op(A) op(B).
-__global__ void __launch_bounds__(NT) cgemm_kernel(big::Common c, LargeOps d, GemmJob job, const float2* ext_in,
-                                                   float2* ext_out) {
-  __shared__ float2 As[BK * (BM + 1)];
-  __shared__ float2 Bs[BK * (BN + 1)];
+// grid (tiles * tiles, 1, B * Kz): one tile of C = sum_terms alpha op(A) op(B), each term
+// summed by ascending k and then added.  Two slices are in flight while one is multiplied.
+template <int R>
+__global__ void __launch_bounds__(NT, R <= 2 ? 4 : (R == 3 ? 3 : (R == 4 ? 2 : 1))) cgemm_kernel(big::Common c, LargeOps d, GemmJob job,
+                                                                   const float2* ext_in, float2* ext_out) {
+  using Ti = Tile<R>;
+  extern __shared__ float2 ring[];
+  __shared__ TermPtrs terms[4];
+  __shared__ int nterms_sh;
   const int n = d.n;
   const int Kz = job.kdst < 0 ? d.K : 1;
   const int b = blockIdx.z / Kz;
@@ -160,83 +199,66 @@ __global__ void __launch_bounds__(NT) cgemm_kernel(big::Common c, LargeOps d, Ge
   if (job_skips(c, b, job.need_run, job.kry) || banded(d, b)) return;
   const int Kb = jumps_of(d, b);
   if (job.kdst < 0 && kz >= Kb) return;  // this instance has fewer jumps
-  const int tiles = (n + BM - 1) / BM;
-  const int tr = blockIdx.x / tiles, tc = blockIdx.x % tiles;
-  const int r0 = tr * BM, c0 = tc * BN;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  float2 acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
-
-  for (int t = 0; t < job.nterms; ++t) {
-    const Term T = job.t[t];
-    if ((T.srcA == SRC_T || T.srcA == SRC_L) && T.kA >= Kb) continue;  // missing jump
-    const float2* A = src_ptr(c, d, b, T.srcA, T.kA < 0 ? kz : T.kA, job.in_sel, ext_in);
-    const float2* B = src_ptr(c, d, b, T.srcB, T.kB < 0 ? kz : T.kB, job.in_sel, ext_in);
-    float2 ra[4], rb[4];
-    float2 tsum[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) tsum[i][j] = make_float2(0.f, 0.f);
-    for (int k0 = 0; k0 < n; k0 += BK) {
-      load_slice(ra, A, n, r0, k0, T.opA);
-      // op(B)[k][col]: op 0 -> B[k][col]; op 1 -> conj(B[col][k]).  Load into Bs[k][col].
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int e = threadIdx.x + q * NT;
-        int col, k;
-        if (T.opB == 0) {
-          k = e / BN;
-          col = e % BN;
-        } else {
-          col = e / BK;
-          k = e % BK;
-        }
-        const int gc = c0 + col, gk = k0 + k;
-        float2 v = make_float2(0.f, 0.f);
-        if (gc < n && gk < n) v = T.opB == 0 ? B[(long long)gk * n + gc] : cconj(B[(long long)gc * n + gk]);
-        rb[q] = v;
-      }
-      __syncthreads();
-      store_slice(As, ra, T.opA);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int e = threadIdx.x + q * NT;
-        int col, k;
-        if (T.opB == 0) {
-          k = e / BN;
-          col = e % BN;
-        } else {
-          col = e / BK;
-          k = e % BK;
-        }
-        Bs[k * (BN + 1) + col] = rb[q];
-      }
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < BK; ++k) {
-        float2 a[4], bb[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = As[k * (BM + 1) + ty + 16 * i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bb[j] = Bs[k * (BN + 1) + tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) cmac(tsum[i][j], a[i], bb[j]);
-      }
+  if (threadIdx.x == 0) {
+    int nt = 0;
+    for (int t = 0; t < job.nterms; ++t) {
+      const Term T = job.t[t];
+      if ((T.srcA == SRC_T || T.srcA == SRC_L) && T.kA >= Kb) continue;  // missing jump
+      terms[nt].A = src_ptr(c, d, b, T.srcA, T.kA < 0 ? kz : T.kA, job.in_sel, ext_in);
+      terms[nt].B = src_ptr(c, d, b, T.srcB, T.kB < 0 ? kz : T.kB, job.in_sel, ext_in);
+      terms[nt].opA = T.opA;
+      terms[nt].opB = T.opB;
+      terms[nt++].alpha = T.alpha;
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        acc[i][j].x = fmaf(T.alpha, tsum[i][j].x, acc[i][j].x);
-        acc[i][j].y = fmaf(T.alpha, tsum[i][j].y, acc[i][j].y);
-      }
+    nterms_sh = nt;
   }
+  __syncthreads();
+  const int tiles = (n + Ti::T - 1) / Ti::T;
+  const int r0 = (int)(blockIdx.x / tiles) * Ti::T, c0 = (int)(blockIdx.x % tiles) * Ti::T;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int slices = (n + BK - 1) / BK, total = nterms_sh * slices;
+  float2 acc[R][R], tsum[R][R];
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < R; ++j) acc[i][j] = tsum[i][j] = make_float2(0.f, 0.f);
+
+  int ft = 0, fs = 0;  // term and slice of the next copy
+  auto fetch = [&](int it) {
+    if (it < total) {
+      const TermPtrs& P = terms[ft];
+      float2* S = ring + (it % kRing) * 2 * Ti::kOperand;
+      copy_slice<R>(S, P.A, n, r0, fs * BK, P.opA != 0);
+      copy_slice<R>(S + Ti::kOperand, P.B, n, c0, fs * BK, P.opB == 0);
+      if (++fs == slices) fs = 0, ++ft;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int it = 0; it < kRing - 1; ++it) fetch(it);
+  int t = 0, sl = 0;
+  for (int it = 0; it < total; ++it) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory");
+    __syncthreads();  // slice `it` has landed for every thread, slice it - 1 has been used
+    fetch(it + kRing - 1);
+    const float2* S = ring + (it % kRing) * 2 * Ti::kOperand;
+    const TermPtrs& P = terms[t];
+    if (P.opA) mac_slice<R, true, false>(tsum, S, S + Ti::kOperand);  // (op A = ^+ only with op B = 1)
+    else if (P.opB) mac_slice<R, false, true>(tsum, S, S + Ti::kOperand);
+    else mac_slice<R, false, false>(tsum, S, S + Ti::kOperand);
+    if (++sl == slices) {
+      const float alpha = P.alpha;
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          acc[i][j] = caxpy(alpha, tsum[i][j], acc[i][j]);
+          tsum[i][j] = make_float2(0.f, 0.f);
+        }
+      sl = 0;
+      ++t;
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   // epilogue
   float2* C;
   if (ext_out) {
@@ -250,11 +272,11 @@ __global__ void __launch_bounds__(NT) cgemm_kernel(big::Common c, LargeOps d, Ge
   }
   const float2* Hm = job.add_miH ? src_ptr(c, d, b, SRC_H, 0, 0, nullptr) : nullptr;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < R; ++i) {
     const int gr = r0 + ty + 16 * i;
     if (gr >= n) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < R; ++j) {
       const int gc = c0 + tx + 16 * j;
       if (gc >= n) continue;
       float2 v = acc[i][j];
@@ -266,6 +288,49 @@ __global__ void __launch_bounds__(NT) cgemm_kernel(big::Common c, LargeOps d, Ge
       }
       C[(long long)gr * n + gc] = v;
     }
+  }
+}
+
+template <int R>
+void launch_cgemm_tile(cudaStream_t s, const big::Common& c, const LargeOps& d, const GemmJob& j, int zdim,
+                       const float2* ext_in, float2* ext_out) {
+  const int t = (d.n + Tile<R>::T - 1) / Tile<R>::T;
+  cgemm_kernel<R><<<dim3(t * t, 1, zdim), NT, Tile<R>::kSmem, s>>>(c, d, j, ext_in, ext_out);
+}
+
+// The tile (16 R square) of an FP32 product.  A CTA's tile takes kAlone[R] when it has an SM
+// for itself and kBusy[R] per tile when several queue on it (measured at n = 256, in units of
+// half a microsecond: one instance, and 256 of them), so the launch takes about the
+// larger of kAlone and kBusy times the tiles of the busiest SM.  Few instances take small
+// tiles (more SMs), large batches 64, and sizes that another tile pads less take that one
+// (n = 151: 160 rows in 80s, 192 in 64s).  Whole right-hand sides with their set-up, in us,
+// the 64 tile of a synchronous kernel before against the choice: n = 100, 1 instance 76 -> 44;
+// n = 66, 64 instances 98 -> 70; n = 151, 32 instances 172 -> 149; n = 256, 64 instances
+// 1508 -> 1477, 1 instance 217 -> 103.
+int cgemm_tile(int n, int zdim) {
+  constexpr int kSizes = 4;
+  constexpr int kR[kSizes] = {2, 3, 4, 5}, kAlone[kSizes] = {29, 46, 66, 97}, kBusy[kSizes] = {20, 36, 60, 97};
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  sms = std::max(sms, 1);
+  long long best = 0;
+  int r = 4;
+  for (int i = 0; i < kSizes; ++i) {
+    const long long t = (n + 16 * kR[i] - 1) / (16 * kR[i]), per_sm = (t * t * zdim + sms - 1) / sms;
+    const long long cost = std::max<long long>(kAlone[i], per_sm * kBusy[i]);
+    if (best == 0 || cost < best) best = cost, r = kR[i];
+  }
+  return r;
+}
+
+void launch_cgemm(cudaStream_t s, const big::Common& c, const LargeOps& d, const GemmJob& j, int zdim,
+                  const float2* ext_in, float2* ext_out) {
+  switch (cgemm_tile(d.n, zdim)) {
+    case 2: launch_cgemm_tile<2>(s, c, d, j, zdim, ext_in, ext_out); break;
+    case 3: launch_cgemm_tile<3>(s, c, d, j, zdim, ext_in, ext_out); break;
+    case 5: launch_cgemm_tile<5>(s, c, d, j, zdim, ext_in, ext_out); break;
+    default: launch_cgemm_tile<4>(s, c, d, j, zdim, ext_in, ext_out); break;
   }
 }
 
@@ -1066,8 +1131,7 @@ void launch_gemm(cudaStream_t s, const big::Common& c, const LargeOps& d, const 
     else
       launch_tc<64>(s, g, c, d, j, ext_in, ext_out);
   } else {
-    const int t = (d.n + BM - 1) / BM;
-    cgemm_kernel<<<dim3(t * t, 1, zdim), NT, 0, s>>>(c, d, j, ext_in, ext_out);
+    launch_cgemm(s, c, d, j, zdim, ext_in, ext_out);
   }
 }
 
@@ -1278,7 +1342,6 @@ void launch_band_setup(cudaStream_t s, const big::Common& c, const LargeOps& d, 
 }
 
 void launch_hnh(cudaStream_t s, const big::Common& c, const LargeOps& d, int B, int need_run) {
-  const int tiles = (d.n + BM - 1) / BM;
   GemmJob j;
   std::memset(&j, 0, sizeof(j));
   j.dst = SRC_HNH;
@@ -1290,7 +1353,7 @@ void launch_hnh(cudaStream_t s, const big::Common& c, const LargeOps& d, int B, 
     int nt = 0;
     while (k < d.K && nt < 4) j.t[nt++] = Term{SRC_L, k, 1, SRC_L, k, 0, -0.5f}, ++k;
     j.nterms = nt;
-    cgemm_kernel<<<dim3(tiles * tiles, 1, B), NT, 0, s>>>(c, d, j, nullptr, nullptr);
+    launch_cgemm(s, c, d, j, B, nullptr, nullptr);
     j.add_miH = 0;
     j.accumulate = 1;
   } while (k < d.K);
@@ -1328,7 +1391,6 @@ static void init_carveouts() {
     prefer_max_shared(big::pre_finalize_kernel);
     prefer_max_shared(big::finalize_kernel);
     prefer_max_shared(zero_words_kernel);
-    prefer_max_shared(cgemm_kernel);
     prefer_max_shared(symmetrize_kernel);
     prefer_max_shared(band_rhs_kernel<true>);
     prefer_max_shared(band_rhs_kernel<false>);
@@ -1338,16 +1400,20 @@ static void init_carveouts() {
     prefer_max_shared(choose_loop_kernel);
     prefer_max_shared(hnh_td_dense_kernel);
     prefer_max_shared(lt_td_dense_kernel);
-    auto tc_attrs = [](auto kern, int smem) {
+    auto dyn_attrs = [](auto kern, int smem) {
       prefer_max_shared(kern);
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     };
-    tc_attrs(tc_cgemm_kernel<DQB_PREC_TF32X3, 128>, tcg::Cfg<128>::kSmem);
-    tc_attrs(tc_cgemm_kernel<DQB_PREC_BF16X3, 128>, tcg::Cfg<128>::kSmem);
-    tc_attrs(tc_cgemm_kernel<DQB_PREC_TF32, 128>, tcg::Cfg<128>::kSmem);
-    tc_attrs(tc_cgemm_kernel<DQB_PREC_TF32X3, 64>, tcg::Cfg<64>::kSmem);
-    tc_attrs(tc_cgemm_kernel<DQB_PREC_BF16X3, 64>, tcg::Cfg<64>::kSmem);
-    tc_attrs(tc_cgemm_kernel<DQB_PREC_TF32, 64>, tcg::Cfg<64>::kSmem);
+    dyn_attrs(cgemm_kernel<2>, Tile<2>::kSmem);
+    dyn_attrs(cgemm_kernel<3>, Tile<3>::kSmem);
+    dyn_attrs(cgemm_kernel<4>, Tile<4>::kSmem);
+    dyn_attrs(cgemm_kernel<5>, Tile<5>::kSmem);
+    dyn_attrs(tc_cgemm_kernel<DQB_PREC_TF32X3, 128>, tcg::Cfg<128>::kSmem);
+    dyn_attrs(tc_cgemm_kernel<DQB_PREC_BF16X3, 128>, tcg::Cfg<128>::kSmem);
+    dyn_attrs(tc_cgemm_kernel<DQB_PREC_TF32, 128>, tcg::Cfg<128>::kSmem);
+    dyn_attrs(tc_cgemm_kernel<DQB_PREC_TF32X3, 64>, tcg::Cfg<64>::kSmem);
+    dyn_attrs(tc_cgemm_kernel<DQB_PREC_BF16X3, 64>, tcg::Cfg<64>::kSmem);
+    dyn_attrs(tc_cgemm_kernel<DQB_PREC_TF32, 64>, tcg::Cfg<64>::kSmem);
   });
 }
 

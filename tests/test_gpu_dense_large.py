@@ -162,3 +162,37 @@ def test_large_path_krylov_standard_form(cuda_device):
     m = dq.Tsit5()
     assert_solve_parity(res.states.cpu().numpy(), None, int(res.infos.nsteps), H, Ls, rho, ts,
                         None, 'Tsit5', m.rtol, m.atol, form='standard')
+
+
+@pytest.mark.parametrize('n', [65, 79, 80, 81, 95, 96, 97, 129, 159, 161])  # edges of 32..80 tiles
+@pytest.mark.parametrize('batch', [1, 40, 300])  # tile choices: alone, queued, saturated
+@pytest.mark.parametrize('form', [0, 1])
+def test_rhs_product_tiles(cuda_device, n, batch, form):
+    """Every tile size and ragged edge of the FP32 product against complex128 products; the
+    bound is 4 sums of n terms of unit size in FP32."""
+    import ctypes
+
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(n)
+    K = 2
+    cplx = lambda *s: torch.randn(*s, dtype=torch.complex64, generator=g) / n ** 0.5  # noqa: E731
+    H, L, X = cplx(2, n, n), cplx(1, K, n, n), cplx(batch, n, n)
+    H = (H + H.mH) / 2
+    X = (X + X.mH) / 2
+    dev = [x.to(cuda_device) for x in (H, L, X)]
+    idx = torch.arange(batch, dtype=torch.int32, device=cuda_device) % 2
+    zero = torch.zeros(batch, dtype=torch.int32, device=cuda_device)
+    out = torch.empty_like(dev[2])
+    p = _lib.DenseProblem(n=n, n_jumps=K, batch=batch, H=dev[0].data_ptr(), L=dev[1].data_ptr(),
+                          H_index=idx.data_ptr(), L_index=zero.data_ptr())
+    size = lib.dqb_mesolve_dense_large_workspace_size(n, K, 0, 1, batch)
+    ws = torch.empty(size, dtype=torch.uint8, device=cuda_device)
+    rc = lib.dqb_lindblad_rhs_dense_large(ctypes.byref(p), form, dev[2].data_ptr(), out.data_ptr(), ws.data_ptr(),
+                                          size, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    h, ls, x = (v.to(torch.complex128) for v in dev)
+    x = x.clone()
+    A = -1j * h[idx.long()] - 0.5 * sum(l.mH @ l for l in ls[0])
+    ref = A @ x + x @ A.mH + sum(l @ x @ l.mH for l in ls[0])
+    err = torch.linalg.norm(out.to(torch.complex128) - ref) / torch.linalg.norm(ref)
+    assert err <= 4 * n ** 0.5 * 2 ** -24
