@@ -646,10 +646,23 @@ class MESolveB200Integrator:
         ||rho - rho^+||_F / ||rho||_F of every saved state (FP64, on the device)."""
         import torch
 
-        st = states.to(torch.complex128)
-        den = torch.linalg.norm(st.reshape(*st.shape[:-2], -1), dim=-1)
-        num = torch.linalg.norm((st - st.mH).reshape(*st.shape[:-2], -1), dim=-1)
-        return {'trace': trace, 'hermiticity': num / torch.clamp(den, min=1e-300)}
+        n = states.shape[-1]
+        if states.requires_grad or states.dtype != torch.complex64 or states.numel() == 0:
+            st = states.to(torch.complex128)
+            den = torch.linalg.norm(st.reshape(*st.shape[:-2], -1), dim=-1)
+            num = torch.linalg.norm((st - st.mH).reshape(*st.shape[:-2], -1), dim=-1)
+            return {'trace': trace, 'hermiticity': num / torch.clamp(den, min=1e-300)}
+        # (a transposed view, as the vectorized form returns, has the same defect)
+        st = states if states.is_contiguous() else states.transpose(-1, -2).contiguous()
+        count = states.numel() // (n * n)
+        lib = _lib.load()
+        out = torch.empty(states.shape[:-2], dtype=torch.float64, device=states.device)
+        size = lib.dqb_state_hermiticity_workspace_size(n, count)
+        ws = torch.empty(size, dtype=torch.uint8, device=states.device)
+        rc = lib.dqb_state_hermiticity(st.data_ptr(), n, count, out.data_ptr(), ws.data_ptr(), size,
+                                       torch.cuda.current_stream(states.device).cuda_stream)
+        _lib.check(rc, 'dqb_state_hermiticity')
+        return {'trace': trace, 'hermiticity': out}
 
     def _result(self, states, expects, infos, status) -> MESolveResult:
         import torch
