@@ -7,7 +7,7 @@ Same signature, argument checks and batching semantics as the reference: ``H`` o
 ``(...H, n, n)``, ``psi0`` ``(...psi0, n, 1)``, ``tsave`` ``(ntsave,)``, ``exp_ops`` a
 list of ``(n, n)``; cartesian batching gives results of shape ``(...H, ...psi0, ...)``,
 flat batching broadcasts ``...H`` against ``...psi0``.  ``method`` is ``Tsit5`` (default)
-or ``Dopri5``.  Three kernels, by size: n <= 128 one warp per instance
+or ``Dopri5``.  By size: n <= 128 one warp (banded ``H``) or one CTA per instance
 (``dqb_sesolve_dense``; sparse-DIA ``H`` is densified); n up to 8192 the batched
 large-problem stepper with a dense ``H`` (``dqb_sesolve_dense_large``) or with ``H`` kept in
 sparse-DIA storage (``dqb_sesolve_dia``).
@@ -44,7 +44,7 @@ def _check_sesolve_args(H, psi0, exp_ops) -> None:
             _check_shape(E, f'exp_ops[{i}]', '(n, n)')
 
 
-# largest n of the warp-per-instance kernel and of the large-problem stepper
+# largest n of the per-instance kernels and of the large-problem stepper
 WARP_MAX_N = 128
 LARGE_MAX_N = 8192
 
@@ -90,11 +90,12 @@ class SESolveB200Integrator:
         self.options = options
         self.H = H
         self.plan = plan
-        # the identity's expectation value <psi|psi> (FP64 sums) is the norm check; with H
-        # in DIA storage (large n) a dense identity would cost more than the solve, so the
-        # norm is taken from the returned states instead
+        # the norm check <psi|psi> at every save point comes from the saved states (FP64
+        # sums); where only the final state is kept, from the identity as one more
+        # expectation operator (n^2 products per save point) -- but with H in DIA storage
+        # (large n) a dense identity would cost more than the solve
         self._n_user_E = len(Es) if Es else 0
-        self._norm_from_states = self.path == 'dia'
+        self._norm_from_states = self.path == 'dia' or bool(options.save_states)
         self.Es = list(Es or []) + ([] if self._norm_from_states
                                     else [np.eye(_shape(H)[-1], dtype=np.complex64)])
 
@@ -205,8 +206,7 @@ class SESolveB200Integrator:
         import torch
 
         if self._norm_from_states:  # (..., nsave): every saved state, or the final one
-            sd = states.to(torch.complex128)
-            checks = {'norm': (sd.abs() ** 2).sum(dim=(-2, -1))}
+            checks = {'norm': torch.view_as_real(states).double().square().sum(dim=(-3, -2, -1))}
         else:
             checks = {'norm': ex[..., self._n_user_E, :].to(torch.complex128).real}
         infos = b['infos'].reshape(*bshape, 3)

@@ -279,3 +279,30 @@ def test_td_dia_sesolve_and_batched_values(cuda_device):
             ref, nsteps, slack = _oracle_td(Hi, psis[j], ts, atol=1e-6)
             assert _rel(res.states[i, j].cpu().numpy(), ref).max() < 1e-5
             assert abs(int(res.infos.nsteps[i, j]) - nsteps) <= slack, (i, j, nsteps, slack)
+
+
+@pytest.mark.parametrize('n', [1, 2, 31, 32, 33, 63, 64, 65, 127, 128])
+@pytest.mark.parametrize('save_states', [True, False])
+def test_banded_and_full_kernels_agree(cuda_device, n, save_states):
+    """A batch of banded Hamiltonians (a warp each) and the same with 1e-25 in every entry (a
+    CTA each), mixed: both sum a row's products by ascending column, so step counts are
+    equal and states agree to the rounding of the dense-output weights."""
+    rng = np.random.default_rng(n)
+    H = np.zeros((4, n, n), complex)
+    for k in (0, 1, 3):
+        if k < n:
+            H += np.stack([np.diag(rng.normal(size=n - k) + 1j * rng.normal(size=n - k), k) for _ in range(4)])
+    H = ((H + np.conj(np.swapaxes(H, -1, -2))) / 2).astype(np.complex64)
+    full = H + np.complex64(1e-25)
+    psi = rng.normal(size=(n, 1)) + 1j * rng.normal(size=(n, 1))
+    psi = (psi / np.linalg.norm(psi)).astype(np.complex64)
+    E = [H[0] / n]
+    opts = dq.Options(save_states=save_states)
+    method = dq.Tsit5(rtol=1e-5, atol=1e-6)
+    got = dq.sesolve(np.stack([H[0], full[1], H[2], full[3]]), psi, [0.0, 0.2, 0.5], exp_ops=E, options=opts, method=method)
+    ref = dq.sesolve(np.stack([full[0], H[1], full[2], H[3]]), psi, [0.0, 0.2, 0.5], exp_ops=E, options=opts, method=method)
+    assert torch.equal(got.infos.nsteps, ref.infos.nsteps)
+    # entries of at most 1, at most ~50 steps: eight roundings
+    assert (got.states - ref.states).abs().amax() <= 8 * 2 ** -24
+    assert (got.expects - ref.expects).abs().amax() <= 1e-6
+    assert (got.checks['norm'] - 1).abs().amax() <= 1e-4
