@@ -29,9 +29,10 @@
 // alike, which needs no barrier.  Two warps per scheduler issue in 40% of the cycles; the
 // rest are fixed latencies, shared-memory waits and instruction fetch.
 //
-// Measured (one B200): driven Kerr, n = 64, two jumps, 1024 instances, t = 1.6: 17.1 ms
-// against 153.4 ms for the product kernel; n = 21, one jump, 1000 instances: 1.55 against
-// 5.31 ms; one n = 16 oscillator with 101 saves: 0.39 against 0.72 ms.
+// Measured (one B200): driven Kerr, n = 64, two jumps, 1024 instances, t = 1.6: 16.9 ms
+// against 153.4 ms for the product kernel; n = 21, one jump, 1000 instances: 1.45 against
+// 5.31 ms; n = 8, 2000 instances: 0.42 against 2.28 ms; one n = 16 oscillator with 101 saves:
+// 0.27 against 0.72 ms (0.38 with one diagonal per pass and registers for four CTAs per SM).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -106,13 +107,18 @@ __host__ __device__ constexpr int dyn_values(bool td) {
 // Sets the bits of M's nonzero diagonals (bit j - i + kMid).
 template <int NT>
 __device__ __forceinline__ void scan_diagonals(const float2* __restrict__ M, int n, unsigned* mask) {
-  for (int e = threadIdx.x; e < n * n; e += NT) {
-    const float2 v = M[e];
-    if (v.x != 0.f || v.y != 0.f) {
-      const int i = e / n, b = e - i * n - i + kMid;
-      const unsigned bit = 1u << (b & 31);
-      if (!(*(volatile unsigned*)&mask[b >> 5] & bit)) atomicOr(&mask[b >> 5], bit);
-    }
+  constexpr int U = 4;  // values in flight per thread
+  for (int e0 = threadIdx.x; e0 < n * n; e0 += U * NT) {
+    float2 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = e0 + u * NT < n * n ? __ldg(M + e0 + u * NT) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (v[u].x != 0.f || v[u].y != 0.f) {
+        const int e = e0 + u * NT, i = e / n, b = e - i * n - i + kMid;
+        const unsigned bit = 1u << (b & 31);
+        if (!(*(volatile unsigned*)&mask[b >> 5] & bit)) atomicOr(&mask[b >> 5], bit);
+      }
   }
 }
 
@@ -176,19 +182,6 @@ __device__ __forceinline__ void block_sums(double (&v)[N], Shared<T, R>& sh, int
   par ^= 1;
 }
 
-// x / y in FP64 where y lies in FP32's normal range: FP32 reciprocal, two Newton steps
-// (relative error below 2^-50); the division otherwise (zero, infinite or NaN y included).
-__device__ __forceinline__ double ratio(double x, double y) {
-  const float f = (float)y;
-  if (f > 1e-30f && f < 1e30f) {
-    double r = (double)__frcp_rn(f);
-    r = fma(r, fma(-y, r, 1.0), r);
-    r = fma(r, fma(-y, r, 1.0), r);
-    return x * r;
-  }
-  return x / y;
-}
-
 // One instance.  Returns false (to every thread) when the instance is not banded or its
 // rho0 not hermitian to rounding: nothing has been written then.  FEAT as in
 // mesolve_small_kernel: 1 = time-dependent H, 2 = gradient tape (rows of tape_np values).
@@ -197,6 +190,7 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
   using G = Geo<T, R>;
   constexpr int NP = G::NP, LD = G::LD, NT = G::NT, Q = G::Q;
   constexpr bool kTd = FEAT == 1, kTape = FEAT == 2;
+  constexpr int kStep = Q <= 3 && !kTd ? 4 : 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tx = tid % T, ty = tid / T;
   const InstView& a = sh.v;
@@ -229,8 +223,8 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
         ld[p * NP + i] = (i < n && j >= 0 && j < n) ? a.L[((long long)k * n + i) * n + j] : make_float2(0.f, 0.f);
       }
   __syncthreads();
-  for (int e = tid; e < ls.nh * NP; e += NT) {  // Hnh[i][i + d]
-    const int q = e / NP, i = e - q * NP, j = i + ls.hoff[q];
+  for (int e = tid; e < kMaxH * NP; e += NT) {  // Hnh[i][i + d]; zeros beyond the last diagonal
+    const int q = e / NP, i = e - q * NP, j = q < ls.nh ? i + ls.hoff[q] : -1;
     float2 v = make_float2(0.f, 0.f);
     const bool in = i < n && j >= 0 && j < n;
     if (in) {
@@ -418,7 +412,7 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
           const double2 c = td_coef(td->term[m], a.inst, ts);
           cm[m] = make_float2((float)c.x, (float)c.y);
         }
-      for (int e = tid; e < ls.nh * NP; e += NT) {
+      for (int e = tid; e < (nh + kStep - 1) / kStep * kStep * NP; e += NT) {
         float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
         for (int m = 0; m < kMaxM; ++m)
@@ -457,19 +451,25 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
         cc[r] = cconj(dc[tx + T * r]);
       }
     };
+    // kStep diagonals per pass: with few elements per thread the reads of several hide one
+    // another's latency (the rows of the table beyond nh are zero; a time-dependent H has no
+    // registers left for it)
 #pragma unroll 1
-    for (int d = 0; d < nh; ++d) {
-      const int off = offset_of(hoffs, d);
-      coefs(hq + d * NP, hq + d * NP);
-      displaced(off, off);
-      int q = 0;
+    for (int d0 = 0; d0 < nh; d0 += kStep) {
 #pragma unroll
-      for (int r = 0; r < R; ++r)
+      for (int dd = 0; dd < kStep; ++dd) {
+        const int d = d0 + dd, off = offset_of(hoffs, d);
+        coefs(hq + d * NP, hq + d * NP);
+        displaced(off, off);
+        int q = 0;
 #pragma unroll
-        for (int c = r; c < R; ++c, ++q) {
-          A[q] = cfma(cr[r], X[xr[r] + tx + T * c], A[q]);
-          B[q] = cfma(cc[c], X[xc[c] + (ty + T * r) * LD], B[q]);
-        }
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int c = r; c < R; ++c, ++q) {
+            A[q] = cfma(cr[r], X[xr[r] + tx + T * c], A[q]);
+            B[q] = cfma(cc[c], X[xc[c] + (ty + T * r) * LD], B[q]);
+          }
+      }
     }
 #pragma unroll 1
     for (int jk = 0; jk < nk; ++jk) {
@@ -770,10 +770,11 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
   return true;
 }
 
-// Resident CTAs that the register budget is set for: the elements of a thread decide.
+// Resident CTAs that the register budget is set for: the elements of a thread decide (and
+// T = 16 runs n <= 32 for at most two instances per SM).
 template <int T, int R>
 constexpr int min_ctas() {
-  return T == 16 ? (R == 1 ? 4 : (R == 2 ? 2 : 1)) : (R == 1 ? 16 : (R == 2 ? 10 : (R == 3 ? 6 : 4)));
+  return T == 16 ? (R <= 2 ? 2 : 1) : (R == 1 ? 12 : (R == 2 ? 8 : (R == 3 ? 6 : 4)));
 }
 
 template <int T, int R, int FEAT, bool RAG>

@@ -27,9 +27,9 @@
 //
 // Bound: band_kernel by the latency of the longest instance's steps (their FP64 controller
 // above all), full_kernel by shared-memory bandwidth (n^2 values of the operator per product).
-// Measured (one B200), kernels alone: n = 64 driven Kerr, 1500 instances: 0.96 ms against
+// Measured (one B200), kernels alone: n = 64 driven Kerr, 1500 instances: 0.77 ms against
 // 2.57 ms for one kernel with a warp and a 33 KB tile per instance (six per SM); n = 101 full,
-// 400 instances: 0.77 against 2.12 ms (one 132 KB tile, so one warp, per SM).
+// 400 instances: 0.75 against 2.12 ms (one 132 KB tile, so one warp, per SM).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -99,17 +99,26 @@ struct BandOp {
   int ld, nd;
   unsigned long long off;  // one signed 16-bit value each in two words: |off| < 128
   unsigned long long off_hi;
-  __device__ int offset(int q) const { return (int)(short)((q < 4 ? off : off_hi) >> (16 * (q & 3))); }
   template <int R>
   __device__ __forceinline__ void mul(const float2* sx, int n, int rank, int size, float2 (&acc)[R]) const {
+    // four diagonals per pass, all their reads in flight (the table's rows beyond nd are zero)
 #pragma unroll 1
-    for (int q = 0; q < nd; ++q) {
-      const int o = offset(q);
+    for (int q0 = 0; q0 < nd; q0 += 4) {
+      float2 c[4][R], x[4][R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int i = rank + size * r;  // beyond the matrix the coefficient is zero, any entry will do
-        cmac(acc[r], d[q * ld + i], sx[min(max(i + o, 0), n - 1)]);
+      for (int q = 0; q < 4; ++q) {
+        const int o = (int)(short)((q0 == 0 ? off : off_hi) >> (16 * q));
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int i = rank + size * r;  // beyond the matrix the coefficient is zero, any entry will do
+          c[q][r] = d[(q0 + q) * ld + i];
+          x[q][r] = sx[min(max(i + o, 0), n - 1)];
+        }
       }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int r = 0; r < R; ++r) cmac(acc[r], c[q][r], x[q][r]);
     }
   }
 };
@@ -299,7 +308,7 @@ __device__ void solve_instance(const Args& a, long long inst, const Op& A, TeamT
       }
       const float ya = cabsf(y[r]), y1a = cabsf(y1[r]);
       const double sc = o.atol + o.rtol * (double)(ya > y1a ? ya : y1a);
-      if (rank + size * r < n) se += (ex * ex + ey * ey) / (sc * sc);
+      if (rank + size * r < n) se += ratio(ex * ex + ey * ey, sc * sc);
     }
     se = tm.sum(se);
     const double err = sqrt(se * inv_n);
@@ -382,17 +391,26 @@ __global__ void __launch_bounds__(32) band_kernel(Args a) {
     if (lane < 8) mask[lane] = 0u;
     __syncwarp();
     // nonzero diagonals (bit j - i + n - 1)
-    for (int i = 0; i < n; ++i)
+    constexpr int U = 8 / R;  // rows in flight
+    for (int i0 = 0; i0 < n; i0 += U) {
+      float2 e[U][R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int j = lane + 32 * r;
-        if (j >= n) continue;
-        const float2 e = __ldg(H + (long long)i * n + j);
-        if (e.x != 0.f || e.y != 0.f) {
-          const int b = j - i + n - 1;
-          if (!(*(volatile unsigned*)&mask[b >> 5] >> (b & 31) & 1u)) atomicOr(&mask[b >> 5], 1u << (b & 31));
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int i = i0 + u, j = lane + 32 * r;
+          e[u][r] = (i < n && j < n) ? __ldg(H + (long long)i * n + j) : make_float2(0.f, 0.f);
         }
-      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (e[u][r].x != 0.f || e[u][r].y != 0.f) {
+            const int b = lane + 32 * r - (i0 + u) + n - 1;
+            if (!(*(volatile unsigned*)&mask[b >> 5] >> (b & 31) & 1u)) atomicOr(&mask[b >> 5], 1u << (b & 31));
+          }
+    }
+    for (int e = lane; e < kMaxH * NP; e += 32) sd[e] = make_float2(0.f, 0.f);
     __syncwarp();
     BandOp A;
     A.d = sd;
