@@ -752,6 +752,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) mesolve_adjoint_kernel(AdjAr
     __syncthreads();
     const long long b = inst_sh;
     if (b >= a.batch) break;
+    if (a.pend && a.pend[b] != band::kPending) {  // the banded kernel has taken it
+      __syncthreads();  // every thread has read inst_sh
+      continue;
+    }
     const InstView v = view_of(a, b);
     const long long nn = (long long)n * n;
     float2* gH = A.grad_H + b * nn;
@@ -772,7 +776,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) mesolve_adjoint_kernel(AdjAr
       lam[e] = g;
     }
     int sp = a.ntsave - 1;  // saves are taken from the last one backwards
-    const int N = A.nacc[b];
+    const int N = min(A.nacc[b], a.tape_cap);
     for (int st = N - 1; st >= 0; --st) {
       const double t = v.tape_t[st], h = v.tape_h[st];
       const float2* y = a.tape_y + (b * (long long)a.tape_cap + st) * NN;
@@ -914,6 +918,301 @@ __global__ void __launch_bounds__(kSmallThreads, 1) mesolve_adjoint_kernel(AdjAr
   }
 }
 
+// ---- banded instances --------------------------------------------------------------------
+// The adjoint of an instance whose operators have few nonzero diagonals (Bands), n <= 48: of
+// the dozen full products of a recorded stage only Zs X and (Zs L_k) X remain, and with them
+// gone the state need not leave the SM: the stage inputs stay in shared memory, the stages
+// and their cotangents in registers (thread (ty, tx) owns elements (ty + 16 r, tx + 16 c)), the
+// operator gradients in registers until the instance ends.  X and Zs are hermitian, so
+// X Zs = (Zs X)^+.  Other instances are marked and left to mesolve_adjoint_kernel.
+// Measured (one B200): driven Kerr, n = 30, one jump, 64 instances: 0.59 against 2.43 ms.
+
+constexpr int kBandDiags = 8;  // diagonals of Hnh, and of the jumps together
+
+struct Bands {
+  unsigned mask[3][4];  // Hnh, L_1, L_2: bit j - i + 63
+  int ok, nh, nl[2];
+  int hoff[kBandDiags], loff[2][kBandDiags];  // ascending
+};
+
+// The nonzero diagonals of Hnh and the jumps (padded, in shared memory); every thread calls it.
+template <int NP>
+__device__ void find_bands(Bands& bl, const float2* sH, const float2* sL, int K) {
+  for (int e = threadIdx.x; e < 12; e += blockDim.x) (&bl.mask[0][0])[e] = 0u;
+  __syncthreads();
+  for (int m = 0; m <= K; ++m) {
+    const float2* M = m == 0 ? sH : sL + (m - 1) * Small<NP>::MAT;
+    for (int e = threadIdx.x; e < NP * NP; e += blockDim.x) {
+      const int i = e / NP, j = e % NP;
+      const float2 v = M[i * Small<NP>::LD + j];
+      if (v.x != 0.f || v.y != 0.f) {
+        const int b = j - i + 63;
+        const unsigned bit = 1u << (b & 31);
+        if (!(*(volatile unsigned*)&bl.mask[m][b >> 5] & bit)) atomicOr(&bl.mask[m][b >> 5], bit);
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    bl.ok = 1;
+    for (int m = 0; m <= K; ++m) {
+      int cnt = 0;
+      for (int w = 0; w < 4; ++w)
+        for (unsigned x = bl.mask[m][w]; x; x &= x - 1) {
+          if (cnt == kBandDiags) {
+            bl.ok = 0;
+            break;
+          }
+          (m == 0 ? bl.hoff : bl.loff[m - 1])[cnt++] = 32 * w + __ffs((int)x) - 1 - 63;
+        }
+      (m == 0 ? bl.nh : bl.nl[m - 1]) = cnt;
+    }
+  }
+  __syncthreads();
+}
+
+// acc += op(A) X (left) or X op(A), A banded (offsets off[0..nd)); op(A) = A^+ when dag.  Sums
+// by ascending inner index, as gemm.
+template <int NP>
+__device__ __forceinline__ void band_mul(float2 (&acc)[NP / 16][NP / 16], const float2* __restrict__ A,
+                                         const float2* __restrict__ X, const int* off, int nd, bool left, bool dag) {
+  constexpr int R = NP / 16, LD = Small<NP>::LD;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  // the inner index is line + o, line the row (left) or column of the result; A[line][line + o]
+  // (left A, or X A^+) ascends with o, A[line - o][line] (left A^+, or X A) with -o
+  const bool rows = left != dag;
+#pragma unroll 1
+  for (int d = 0; d < nd; ++d) {
+    const int o = rows ? off[d] : -off[nd - 1 - d];
+    float2 a[R];
+    int m[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int line = (left ? ty : tx) + 16 * r, in = line + o;
+      m[r] = min(max(in, 0), NP - 1);
+      a[r] = rows ? A[line * LD + m[r]] : A[m[r] * LD + line];
+      if (in != m[r]) a[r] = make_float2(0.f, 0.f);
+      if (dag) a[r].y = -a[r].y;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < R; ++c)
+        acc[r][c] = left ? cfma(a[r], X[m[r] * LD + tx + 16 * c], acc[r][c])
+                         : cfma(X[(ty + 16 * r) * LD + m[c]], a[c], acc[r][c]);
+  }
+}
+
+// acc = S(X), or S^+(X) when dag (the standard form); sT: product buffer.  The caller's
+// barrier before it makes X visible; ends without one.
+template <int NP>
+__device__ __forceinline__ void band_rhs(float2 (&acc)[NP / 16][NP / 16], const float2* sH, const float2* sL,
+                                         const float2* X, float2* sT, const Bands& bl, int K, bool dag) {
+  zero_tile<NP>(acc);
+  band_mul<NP>(acc, sH, X, bl.hoff, bl.nh, true, dag);
+  band_mul<NP>(acc, sH, X, bl.hoff, bl.nh, false, !dag);
+  for (int k = 0; k < K; ++k) {
+    const float2* Lk = sL + k * Small<NP>::MAT;
+    float2 t[NP / 16][NP / 16];
+    zero_tile<NP>(t);
+    band_mul<NP>(t, Lk, X, bl.loff[k], bl.nl[k], true, dag);
+    __syncthreads();  // readers of the previous T are done
+    store_tile<NP>(sT, t, 1.0f);
+    __syncthreads();
+    band_mul<NP>(acc, Lk, sT, bl.loff[k], bl.nl[k], false, !dag);
+  }
+}
+
+// KR: jump operators that it takes at most.  tape_np: row length of the tape's states.
+template <int NP, int KR>
+__global__ void __launch_bounds__(kSmallThreads, NP <= 16 ? 2 : 1) mesolve_adjoint_band_kernel(AdjArgs A, int tape_np,
+                                                                                              int* marks) {
+  extern __shared__ float4 smem_raw[];
+  __shared__ long long inst_sh;
+  __shared__ Bands bl;
+  constexpr int R = NP / 16, LD = Small<NP>::LD, MAT = Small<NP>::MAT;
+  const DenseSmallArgs& a = A.p;
+  const int tid = threadIdx.x, n = a.n, K = a.K;
+  const int tx = tid & 15, ty = tid >> 4;
+  float2* sH = reinterpret_cast<float2*>(smem_raw);
+  float2* sX = sH + MAT;       // X_1..7
+  float2* sZ = sX + 7 * MAT;
+  float2* sT = sZ + MAT;
+  float2* sU = sT + MAT;
+  float2* sL = sU + MAT;
+  const Tableau& T = c_tab[a.o.method];
+  auto each = [&](auto f) {  // f(r, c, i, j) on the thread's elements
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < R; ++c) f(r, c, ty + 16 * r, tx + 16 * c);
+  };
+  for (;;) {
+    if (tid == 0) inst_sh = (long long)atomicAdd(a.counter, 1u);
+    __syncthreads();
+    const long long b = inst_sh;
+    if (b >= a.batch) break;
+    const InstView v = view_of(a, b);
+    const long long nn = (long long)n * n;
+    load_padded<NP>(sH, v.H, n);
+    for (int k = 0; k < K; ++k) load_padded<NP>(sL + k * MAT, v.L + (long long)k * nn, n);
+    __syncthreads();
+    build_hnh<NP>(sH, sL, n, K);
+    __syncthreads();
+    find_bands<NP>(bl, sH, sL, K);
+    if (tid == 0) marks[b] = bl.ok ? 0 : band::kPending;
+    if (!bl.ok) continue;  // (every thread reads bl.ok before the next instance's barriers)
+    const int nsave = a.o.save_states ? a.ntsave : 1;
+    float2 lam[R][R], gH[R][R], gL[KR][R][R];
+    zero_tile<NP>(gH);
+#pragma unroll
+    for (int k = 0; k < KR; ++k) zero_tile<NP>(gL[k]);
+    each([&](int r, int c, int i, int j) {
+      lam[r][c] = make_float2(0.f, 0.f);
+      if (!a.o.save_states && A.gstates && i < n && j < n) lam[r][c] = A.gstates[b * nn + i * n + j];
+    });
+    // cotangent of save point sp on element (i, j)
+    auto save_cot = [&](int sp, int i, int j) {
+      float2 g = make_float2(0.f, 0.f);
+      if (i >= n || j >= n) return g;
+      if (a.o.save_states && A.gstates) g = A.gstates[(b * nsave + sp) * nn + i * n + j];
+      if (A.gexpects)
+        for (int m = 0; m < a.nE; ++m)  // d tr(E rho) / d rho: cotangent ebar E^+
+          g = cfma(A.gexpects[(b * a.nE + m) * a.ntsave + sp], cconj(a.E[((long long)m * n + j) * n + i]), g);
+      return g;
+    };
+    int sp = a.ntsave - 1;  // saves are taken from the last one backwards
+    const int N = min(A.nacc[b], a.tape_cap);
+    for (int st = N - 1; st >= 0; --st) {
+      const double t = v.tape_t[st], h = v.tape_h[st];
+      const float2* Y = a.tape_y + (b * (long long)a.tape_cap + st) * tape_np * tape_np;
+      // (a) the forward stages again: X_1 = y, X_j = y + h sum_{l<j} a_jl k_l, k_j = S(X_j)
+      {
+        float2 y[R][R], ks[6][R][R];
+        each([&](int r, int c, int i, int j) { y[r][c] = Y[i * tape_np + j]; });
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+          float2* X = sX + q * MAT;
+          float cf[6];
+#pragma unroll
+          for (int l = 0; l < 6; ++l) cf[l] = (float)(h * T.a[q][l]);
+          each([&](int r, int c, int i, int j) {
+            float2 x = y[r][c];
+#pragma unroll
+            for (int l = 0; l < 6; ++l)
+              if (l < q) x = caxpy(cf[l], ks[l][r][c], x);
+            X[i * LD + j] = x;
+          });
+          __syncthreads();
+          if (q < 6) band_rhs<NP>(ks[q], sH, sL, X, sT, bl, K, false);
+        }
+      }
+      // (b) direct cotangents of the stages: the step's end state and its saves (after (a), whose
+      // stages want the registers)
+      float2 kap[7][R][R];
+#pragma unroll
+      for (int q = 0; q < 7; ++q) {
+        const float hb = (float)(h * T.b[q]);
+        each([&](int r, int c, int, int) { kap[q][r][c] = make_float2(hb * lam[r][c].x, hb * lam[r][c].y); });
+      }
+      while (sp >= 0 && (st == 0 || a.tsave[sp] > t)) {
+        double w[7];
+        dense_weights(a.o.method, h > 0.0 ? (a.tsave[sp] - t) / h : 1.0, w);
+        each([&](int r, int c, int i, int j) {
+          const float2 g = save_cot(sp, i, j);
+#pragma unroll
+          for (int q = 0; q < 7; ++q) kap[q][r][c] = caxpy((float)(h * w[q]), g, kap[q][r][c]);
+          lam[r][c] = cadd(lam[r][c], g);
+        });
+        --sp;
+      }
+      // (c) stages backwards
+#pragma unroll
+      for (int q = 6; q >= 0; --q) {
+        const float2* X = sX + q * MAT;
+        __syncthreads();  // the previous stage has read sZ, sT and sU
+        store_tile<NP>(sZ, kap[q], 1.0f);
+        __syncthreads();
+        float2 acc[R][R];
+        band_rhs<NP>(acc, sH, sL, sZ, sT, bl, K, true);  // xi = S^+(kappa)
+        each([&](int r, int c, int, int) {
+          lam[r][c] = cadd(lam[r][c], acc[r][c]);
+#pragma unroll
+          for (int l = 0; l < 6; ++l)
+            if (l < q) kap[l][r][c] = caxpy((float)(h * T.a[q][l]), acc[r][c], kap[l][r][c]);
+        });
+        __syncthreads();  // sT has been read
+        each([&](int r, int c, int i, int j) {  // Zs = kappa + kappa^+
+          sT[i * LD + j] = cadd(kap[q][r][c], cconj(sZ[j * LD + i]));
+        });
+        __syncthreads();
+        zero_tile<NP>(acc);
+        gemm<NP, false, false>(acc, sT, X, n);  // Zs X
+        each([&](int r, int c, int, int) { gH[r][c] = cadd(gH[r][c], make_float2(-acc[r][c].y, acc[r][c].x)); });
+        if (K == 0) continue;
+        // G = Zs X + X Zs into sZ
+        store_tile<NP>(sU, acc, 1.0f);
+        __syncthreads();
+        each([&](int r, int c, int i, int j) { sZ[i * LD + j] = cadd(acc[r][c], cconj(sU[j * LD + i])); });
+#pragma unroll
+        for (int k = 0; k < KR; ++k) {
+          if (k >= K) break;
+          const float2* Lk = sL + k * MAT;
+          float2 u[R][R];
+          zero_tile<NP>(u);
+          band_mul<NP>(u, Lk, sT, bl.loff[k], bl.nl[k], false, false);  // Zs L
+          __syncthreads();  // sU has been read, sZ is complete
+          store_tile<NP>(sU, u, 1.0f);
+          zero_tile<NP>(u);
+          band_mul<NP>(u, Lk, sZ, bl.loff[k], bl.nl[k], true, false);  // L G
+          each([&](int r, int c, int, int) { gL[k][r][c] = caxpy(-0.5f, u[r][c], gL[k][r][c]); });
+          __syncthreads();
+          zero_tile<NP>(u);
+          gemm<NP, false, false>(u, sU, X, n);  // (Zs L) X
+          each([&](int r, int c, int, int) { gL[k][r][c] = cadd(gL[k][r][c], u[r][c]); });
+        }
+      }
+      __syncthreads();  // sX has been read
+    }
+    // saves at or before t0 (no step reached them): they read y0 itself
+    for (; sp >= 0; --sp) each([&](int r, int c, int i, int j) { lam[r][c] = cadd(lam[r][c], save_cot(sp, i, j)); });
+    each([&](int r, int c, int i, int j) {
+      if (i < n && j < n) {
+        A.grad_H[b * nn + i * n + j] = gH[r][c];
+#pragma unroll
+        for (int k = 0; k < KR; ++k)
+          if (k < K) A.grad_L[(b * K + k) * nn + i * n + j] = gL[k][r][c];
+        if (!v.is_ket) A.grad_rho0[b * nn + i * n + j] = lam[r][c];
+      }
+    });
+    __syncthreads();
+    // rho0 = psi psi^+ for a ket: psibar = (lambda + lambda^+) psi
+    if (v.is_ket) {
+      store_tile<NP>(sZ, lam, 1.0f);
+      __syncthreads();
+      for (int i = tid; i < n; i += blockDim.x) {
+        float2 acc = make_float2(0.f, 0.f);
+        for (int j = 0; j < n; ++j) acc = cfma(cadd(sZ[i * LD + j], cconj(sZ[j * LD + i])), v.rho0[j], acc);
+        A.grad_rho0[b * n + i] = acc;
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// Launches it when the instances can be taken (size, jumps, shared memory); `launched` says so.
+template <int NP, int KR>
+static int adjoint_band_launch(const AdjArgs& A, int tape_np, int* marks, cudaStream_t s, bool* launched) {
+  const size_t smem = (size_t)(11 + A.p.K) * Small<NP>::MAT * sizeof(float2);
+  if (A.p.K > KR || smem + 2048 > max_optin_smem()) return DQB_OK;
+  const int per_sm = resident_ctas(mesolve_adjoint_band_kernel<NP, KR>, smem);
+  if (per_sm < 1) return DQB_OK;
+  const long long g = std::min<long long>((long long)per_sm * sm_count(), A.p.batch);
+  mesolve_adjoint_band_kernel<NP, KR><<<(unsigned)g, kSmallThreads, smem, s>>>(A, tape_np, marks);
+  *launched = true;
+  return cudaGetLastError() == cudaSuccess ? DQB_OK : DQB_ERR_CUDA;
+}
+
 template <int NP>
 static size_t adjoint_smem_bytes(int K) {
   return (size_t)(4 + K) * Small<NP>::MAT * sizeof(float2);
@@ -974,6 +1273,9 @@ extern "C" int dqb_mesolve_dense_taped(const dqb_dense_problem* p, const dqb_ode
   return cudaGetLastError() == cudaSuccess ? DQB_OK : DQB_ERR_CUDA;
 }
 
+// One mark per instance (banded, or left to the product kernel), after the work counters.
+static size_t adjoint_marks_bytes(long long batch) { return ((size_t)batch * sizeof(int) + 255) & ~(size_t)255; }
+
 extern "C" size_t dqb_mesolve_dense_adjoint_workspace_size(int32_t n, int32_t n_jumps, int64_t batch) {
   using namespace dqb;
   const int NP = pick_np(n);
@@ -981,7 +1283,7 @@ extern "C" size_t dqb_mesolve_dense_adjoint_workspace_size(int32_t n, int32_t n_
   const size_t smem = (size_t)(4 + n_jumps) * (NP + 1) * NP * sizeof(float2);
   if (smem + 2048 > max_optin_smem()) return 0;
   const long long g = std::min<long long>((long long)sm_count(), batch);
-  return 256 + (size_t)g * kAdjMats * NP * NP * sizeof(float2);
+  return 256 + adjoint_marks_bytes(batch) + (size_t)g * kAdjMats * NP * NP * sizeof(float2);
 }
 
 extern "C" int dqb_mesolve_dense_adjoint(const dqb_dense_problem* p, const dqb_ode_options* o,
@@ -1003,8 +1305,10 @@ extern "C" int dqb_mesolve_dense_adjoint(const dqb_dense_problem* p, const dqb_o
   cudaStream_t s = (cudaStream_t)stream;
   AdjArgs A;
   A.p = make_args(p, o, nullptr);
+  const size_t head = 256 + adjoint_marks_bytes(p->batch);
+  int* marks = (int*)((char*)workspace + 256);
   A.p.counter = (unsigned int*)workspace;
-  A.p.slots = (float2*)((char*)workspace + 256);
+  A.p.slots = (float2*)((char*)workspace + head);
   A.p.tape_t = tape->t;
   A.p.tape_h = tape->h;
   A.p.tape_y = (float2*)tape->y;
@@ -1016,7 +1320,17 @@ extern "C" int dqb_mesolve_dense_adjoint(const dqb_dense_problem* p, const dqb_o
   A.grad_H = (float2*)grads->H;
   A.grad_L = (float2*)grads->L;
   zero_words_kernel<<<1, 64, 0, s>>>((unsigned int*)workspace, 64);
-  const long long max_grid = (long long)((workspace_bytes - 256) / ((size_t)kAdjMats * NP * NP * sizeof(float2)));
+  bool launched = false;
+  if (p->n <= 16) rc = adjoint_band_launch<16, 2>(A, NP, marks, s, &launched);
+  else if (p->n <= 32) rc = adjoint_band_launch<32, 2>(A, NP, marks, s, &launched);
+  else if (p->n <= 48) rc = adjoint_band_launch<48, 1>(A, NP, marks, s, &launched);
+  if (rc) return rc;
+  if (launched) {
+    A.p.counter += 1;
+    A.p.pend = marks;
+    A.p.pend_stride = 1;
+  }
+  const long long max_grid = (long long)((workspace_bytes - head) / ((size_t)kAdjMats * NP * NP * sizeof(float2)));
   switch (NP) {
     case 16: return adjoint_launch<16>(A, s, max_grid);
     case 32: return adjoint_launch<32>(A, s, max_grid);

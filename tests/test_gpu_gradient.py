@@ -169,3 +169,36 @@ def test_gradient_with_batched_jump_operators(cuda_device):
             gH[i] += Hi.grad
     np.testing.assert_allclose(L.grad.numpy(), gL.numpy(), rtol=1e-5, atol=1e-6)
     np.testing.assert_allclose(H.grad.numpy(), gH.numpy(), rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize('n, jumps', [(2, 0), (15, 1), (16, 2), (17, 2), (31, 1), (32, 2), (33, 1), (48, 1)])
+@pytest.mark.parametrize('ket', [True, False])
+def test_banded_adjoint_same_as_products(cuda_device, n, jumps, ket):
+    """The adjoint kernel of banded instances against the product kernel (1e-25 in every entry
+    of H: full matrices, the same solve), in one mixed batch each, at the edges of its sizes.
+    Both sum the same products in FP32; the bound is 64 roundings of the largest gradient."""
+    rng = np.random.default_rng(n)
+    H = np.zeros((2, n, n), complex)
+    for k in (0, 1, 3):
+        if k < n:
+            H += np.stack([np.diag(rng.normal(size=n - k) + 1j * rng.normal(size=n - k), k) for _ in range(2)])
+    H = ((H + np.conj(np.swapaxes(H, -1, -2))) / 2).astype(np.complex64)
+    Ls = [(0.3 * np.diag(rng.normal(size=n - o), o)).astype(np.complex64) for o in (1, 0)[:jumps]]
+    y = rng.normal(size=(n, 1)) + 1j * rng.normal(size=(n, 1))
+    y = y / np.linalg.norm(y)
+    rho = (y if ket else y @ y.conj().T).astype(np.complex64)
+    E = (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))).astype(np.complex64)
+    E = (E + E.conj().T) / 2
+    W = torch.as_tensor(rng.normal(size=(3, n, n)) + 1j * rng.normal(size=(3, n, n)), dtype=torch.complex64)
+
+    def grads(h):
+        leaves = [torch.as_tensor(v).clone().requires_grad_() for v in (h, *Ls, rho)]
+        res = dq.mesolve(leaves[0], leaves[1:-1], leaves[-1], [0.0, 0.1, 0.3], exp_ops=[E])
+        loss = (W.to(res.states.device).conj() * res.states).sum().real + res.expects.real.sum()
+        return torch.autograd.grad(loss, leaves)
+
+    mixed = [H.copy(), H.copy()]
+    mixed[0][1] += np.complex64(1e-25)
+    mixed[1][0] += np.complex64(1e-25)
+    for a, b in zip(grads(mixed[0]), grads(mixed[1])):
+        assert (a - b).abs().max() <= 64 * 2 ** -24 * b.abs().max()
