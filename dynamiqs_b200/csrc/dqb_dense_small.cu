@@ -214,6 +214,126 @@ __device__ void rhs(const float2* sH, const float2* sL, const float2* sX, float2
   }
 }
 
+// ---- products with banded operators -------------------------------------------------------
+// Used where the state is not hermitian by construction -- the standard form and the adjoint --;
+// the hermitian form's banded instances have a kernel of their own (dqb_dense_small_band.cu).
+
+constexpr int kBandDiags = 8;  // diagonals of Hnh, and of the jumps together
+
+struct Bands {
+  unsigned mask[3][4];  // Hnh, L_1, L_2: bit j - i + 63
+  int ok, nh, nl[2];
+  int hoff[kBandDiags], loff[2][kBandDiags];  // ascending
+};
+
+// The nonzero diagonals of Hnh and the jumps (padded, in shared memory); every thread calls it.
+template <int NP>
+__device__ void find_bands(Bands& bl, const float2* sH, const float2* sL, int K) {
+  for (int e = threadIdx.x; e < 12; e += blockDim.x) (&bl.mask[0][0])[e] = 0u;
+  // the nonzeros of one row lie on as many diagonals: full matrices are told by one row
+  const int mid = NP / 2 * Small<NP>::LD + threadIdx.x % NP;
+  if (__syncthreads_count(threadIdx.x < NP && (sH[mid].x != 0.f || sH[mid].y != 0.f)) > kBandDiags) {
+    if (threadIdx.x == 0) bl.ok = 0;
+    __syncthreads();
+    return;
+  }
+  for (int m = 0; m <= K; ++m) {
+    const float2* M = m == 0 ? sH : sL + (m - 1) * Small<NP>::MAT;
+    for (int e = threadIdx.x; e < NP * NP; e += blockDim.x) {
+      const int i = e / NP, j = e % NP;
+      const float2 v = M[i * Small<NP>::LD + j];
+      if (v.x != 0.f || v.y != 0.f) {
+        const int b = j - i + 63;
+        const unsigned bit = 1u << (b & 31);
+        if (!(*(volatile unsigned*)&bl.mask[m][b >> 5] & bit)) atomicOr(&bl.mask[m][b >> 5], bit);
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    bl.ok = 1;
+    for (int m = 0; m <= K; ++m) {
+      int cnt = 0;
+      for (int w = 0; w < 4; ++w)
+        for (unsigned x = bl.mask[m][w]; x; x &= x - 1) {
+          if (cnt == kBandDiags) {
+            bl.ok = 0;
+            break;
+          }
+          (m == 0 ? bl.hoff : bl.loff[m - 1])[cnt++] = 32 * w + __ffs((int)x) - 1 - 63;
+        }
+      (m == 0 ? bl.nh : bl.nl[m - 1]) = cnt;
+    }
+  }
+  __syncthreads();
+}
+
+// acc += op(A) X (left) or X op(A), A banded (offsets off[0..nd)); op(A) = A^+ when dag.  Sums
+// by ascending inner index, as gemm.
+template <int NP>
+__device__ __forceinline__ void band_mul(float2 (&acc)[NP / 16][NP / 16], const float2* __restrict__ A,
+                                         const float2* __restrict__ X, const int* off, int nd, bool left, bool dag) {
+  constexpr int R = NP / 16, LD = Small<NP>::LD;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  // the inner index is line + o, line the row (left) or column of the result; A[line][line + o]
+  // (left A, or X A^+) ascends with o, A[line - o][line] (left A^+, or X A) with -o
+  const bool rows = left != dag;
+#pragma unroll 1
+  for (int d = 0; d < nd; ++d) {
+    const int o = rows ? off[d] : -off[nd - 1 - d];
+    float2 a[R];
+    int m[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int line = (left ? ty : tx) + 16 * r, in = line + o;
+      m[r] = min(max(in, 0), NP - 1);
+      a[r] = rows ? A[line * LD + m[r]] : A[m[r] * LD + line];
+      if (in != m[r]) a[r] = make_float2(0.f, 0.f);
+      if (dag) a[r].y = -a[r].y;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < R; ++c)
+        acc[r][c] = left ? cfma(a[r], X[m[r] * LD + tx + 16 * c], acc[r][c])
+                         : cfma(X[(ty + 16 * r) * LD + m[c]], a[c], acc[r][c]);
+  }
+}
+
+// acc = S(X), or S^+(X) when dag (the standard form); sT: product buffer.  The caller's
+// barrier before it makes X visible; ends without one.
+template <int NP>
+__device__ __forceinline__ void band_rhs(float2 (&acc)[NP / 16][NP / 16], const float2* sH, const float2* sL,
+                                         const float2* X, float2* sT, const Bands& bl, int K, bool dag) {
+  zero_tile<NP>(acc);
+  band_mul<NP>(acc, sH, X, bl.hoff, bl.nh, true, dag);
+  band_mul<NP>(acc, sH, X, bl.hoff, bl.nh, false, !dag);
+  for (int k = 0; k < K; ++k) {
+    const float2* Lk = sL + k * Small<NP>::MAT;
+    float2 t[NP / 16][NP / 16];
+    zero_tile<NP>(t);
+    band_mul<NP>(t, Lk, X, bl.loff[k], bl.nl[k], true, dag);
+    __syncthreads();  // readers of the previous T are done
+    store_tile<NP>(sT, t, 1.0f);
+    __syncthreads();
+    band_mul<NP>(acc, Lk, sT, bl.loff[k], bl.nl[k], false, !dag);
+  }
+}
+
+// out[i * NP + j] = S(X)[i][j], the standard form of a banded instance.  A call and not inlined:
+// its registers then cost the product path none.
+template <int NP>
+__device__ __noinline__ void band_rhs_out(const float2* sH, const float2* sL, const float2* sX, float2* sT,
+                                          const Bands* bl, int K, float2* __restrict__ out) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float2 acc[NP / 16][NP / 16];
+  band_rhs<NP>(acc, sH, sL, sX, sT, *bl, K, false);
+#pragma unroll
+  for (int r = 0; r < NP / 16; ++r)
+#pragma unroll
+    for (int c = 0; c < NP / 16; ++c) out[(ty + 16 * r) * NP + tx + 16 * c] = acc[r][c];
+}
+
 // The right-hand side on CUDA cores (the engine of solve_one, dqb_small.cuh): Hnh, the
 // jump operators, the stage input X and the product buffer T in padded shared memory.
 // With a time-dependent H (td->M > 0) the constant part Hnh0 = -iH0 - 1/2 sum L^+L is kept
@@ -227,6 +347,7 @@ struct SimtEngine {
   const TdArgs* td;
   float2* sH0;
   long long inst;
+  Bands* bl;  // standard form: the banded instances' diagonals
 
   __device__ void load(const InstView& a) {
     n = a.n;
@@ -239,6 +360,11 @@ struct SimtEngine {
     __syncthreads();
     if constexpr (kJumps) {
       for (int e = threadIdx.x; e < Small<NP>::MAT; e += blockDim.x) sH0[e] = sH[e];
+      __syncthreads();
+    }
+    if constexpr (!kJumps) {
+      if (form == DQB_FORM_STANDARD && K <= 2) find_bands<NP>(*bl, sH, sL, K);
+      else if (threadIdx.x == 0) bl->ok = 0;
       __syncthreads();
     }
   }
@@ -275,7 +401,8 @@ struct SimtEngine {
       }
     }
     __syncthreads();
-    dqb::rhs<NP>(sH, sL, sX, sT, n, K, form, out, NP, NP);
+    if (!kJumps && bl->ok) band_rhs_out<NP>(sH, sL, sX, sT, bl, K, out);
+    else dqb::rhs<NP>(sH, sL, sX, sT, n, K, form, out, NP, NP);
     __syncthreads();
   }
 
@@ -288,6 +415,7 @@ __global__ void __launch_bounds__(kSmallThreads, NP == 64 ? 1 : (NP == 48 ? 2 : 
   extern __shared__ float4 smem_raw[];
   __shared__ double red[40];
   __shared__ Ctrl ctl;
+  __shared__ Bands bl;
   float2* sH = reinterpret_cast<float2*>(smem_raw);
   float2* sX = sH + Small<NP>::MAT;
   float2* sT = sX + Small<NP>::MAT;
@@ -305,7 +433,7 @@ __global__ void __launch_bounds__(kSmallThreads, NP == 64 ? 1 : (NP == 48 ? 2 : 
       continue;
     }
     const InstView v = view_of(a, inst);
-    SimtEngine<NP, FEAT> eng{sH, sX, sT, sL, a.n, a.K, a.o.form, &a.td, sL + a.K * Small<NP>::MAT, inst};
+    SimtEngine<NP, FEAT> eng{sH, sX, sT, sL, a.n, a.K, a.o.form, &a.td, sL + a.K * Small<NP>::MAT, inst, &bl};
     solve_one<NP>(eng, v, a.o, slot, red, ctl);
     __syncthreads();
   }
@@ -927,102 +1055,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) mesolve_adjoint_kernel(AdjAr
 // X Zs = (Zs X)^+.  Other instances are marked and left to mesolve_adjoint_kernel.
 // Measured (one B200): driven Kerr, n = 30, one jump, 64 instances: 0.59 against 2.43 ms.
 
-constexpr int kBandDiags = 8;  // diagonals of Hnh, and of the jumps together
-
-struct Bands {
-  unsigned mask[3][4];  // Hnh, L_1, L_2: bit j - i + 63
-  int ok, nh, nl[2];
-  int hoff[kBandDiags], loff[2][kBandDiags];  // ascending
-};
-
-// The nonzero diagonals of Hnh and the jumps (padded, in shared memory); every thread calls it.
-template <int NP>
-__device__ void find_bands(Bands& bl, const float2* sH, const float2* sL, int K) {
-  for (int e = threadIdx.x; e < 12; e += blockDim.x) (&bl.mask[0][0])[e] = 0u;
-  __syncthreads();
-  for (int m = 0; m <= K; ++m) {
-    const float2* M = m == 0 ? sH : sL + (m - 1) * Small<NP>::MAT;
-    for (int e = threadIdx.x; e < NP * NP; e += blockDim.x) {
-      const int i = e / NP, j = e % NP;
-      const float2 v = M[i * Small<NP>::LD + j];
-      if (v.x != 0.f || v.y != 0.f) {
-        const int b = j - i + 63;
-        const unsigned bit = 1u << (b & 31);
-        if (!(*(volatile unsigned*)&bl.mask[m][b >> 5] & bit)) atomicOr(&bl.mask[m][b >> 5], bit);
-      }
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    bl.ok = 1;
-    for (int m = 0; m <= K; ++m) {
-      int cnt = 0;
-      for (int w = 0; w < 4; ++w)
-        for (unsigned x = bl.mask[m][w]; x; x &= x - 1) {
-          if (cnt == kBandDiags) {
-            bl.ok = 0;
-            break;
-          }
-          (m == 0 ? bl.hoff : bl.loff[m - 1])[cnt++] = 32 * w + __ffs((int)x) - 1 - 63;
-        }
-      (m == 0 ? bl.nh : bl.nl[m - 1]) = cnt;
-    }
-  }
-  __syncthreads();
-}
-
-// acc += op(A) X (left) or X op(A), A banded (offsets off[0..nd)); op(A) = A^+ when dag.  Sums
-// by ascending inner index, as gemm.
-template <int NP>
-__device__ __forceinline__ void band_mul(float2 (&acc)[NP / 16][NP / 16], const float2* __restrict__ A,
-                                         const float2* __restrict__ X, const int* off, int nd, bool left, bool dag) {
-  constexpr int R = NP / 16, LD = Small<NP>::LD;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  // the inner index is line + o, line the row (left) or column of the result; A[line][line + o]
-  // (left A, or X A^+) ascends with o, A[line - o][line] (left A^+, or X A) with -o
-  const bool rows = left != dag;
-#pragma unroll 1
-  for (int d = 0; d < nd; ++d) {
-    const int o = rows ? off[d] : -off[nd - 1 - d];
-    float2 a[R];
-    int m[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int line = (left ? ty : tx) + 16 * r, in = line + o;
-      m[r] = min(max(in, 0), NP - 1);
-      a[r] = rows ? A[line * LD + m[r]] : A[m[r] * LD + line];
-      if (in != m[r]) a[r] = make_float2(0.f, 0.f);
-      if (dag) a[r].y = -a[r].y;
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int c = 0; c < R; ++c)
-        acc[r][c] = left ? cfma(a[r], X[m[r] * LD + tx + 16 * c], acc[r][c])
-                         : cfma(X[(ty + 16 * r) * LD + m[c]], a[c], acc[r][c]);
-  }
-}
-
-// acc = S(X), or S^+(X) when dag (the standard form); sT: product buffer.  The caller's
-// barrier before it makes X visible; ends without one.
-template <int NP>
-__device__ __forceinline__ void band_rhs(float2 (&acc)[NP / 16][NP / 16], const float2* sH, const float2* sL,
-                                         const float2* X, float2* sT, const Bands& bl, int K, bool dag) {
-  zero_tile<NP>(acc);
-  band_mul<NP>(acc, sH, X, bl.hoff, bl.nh, true, dag);
-  band_mul<NP>(acc, sH, X, bl.hoff, bl.nh, false, !dag);
-  for (int k = 0; k < K; ++k) {
-    const float2* Lk = sL + k * Small<NP>::MAT;
-    float2 t[NP / 16][NP / 16];
-    zero_tile<NP>(t);
-    band_mul<NP>(t, Lk, X, bl.loff[k], bl.nl[k], true, dag);
-    __syncthreads();  // readers of the previous T are done
-    store_tile<NP>(sT, t, 1.0f);
-    __syncthreads();
-    band_mul<NP>(acc, Lk, sT, bl.loff[k], bl.nl[k], false, !dag);
-  }
-}
-
 // KR: jump operators that it takes at most.  tape_np: row length of the tape's states.
 template <int NP, int KR>
 __global__ void __launch_bounds__(kSmallThreads, NP <= 16 ? 2 : 1) mesolve_adjoint_band_kernel(AdjArgs A, int tape_np,
@@ -1400,6 +1432,7 @@ __global__ void __launch_bounds__(kSmallThreads, NP == 64 ? 1 : (NP == 32 ? 3 : 
   extern __shared__ float4 smem_raw[];
   __shared__ double red[40];
   __shared__ Ctrl ctl;
+  __shared__ Bands bl;
   float2* sH = reinterpret_cast<float2*>(smem_raw);
   float2* sX = sH + Small<NP>::MAT;
   float2* sT = sX + Small<NP>::MAT;
@@ -1415,7 +1448,7 @@ __global__ void __launch_bounds__(kSmallThreads, NP == 64 ? 1 : (NP == 32 ? 3 : 
       continue;
     }
     const InstView v = view_of_ragged(d[inst], inst);
-    SimtEngine<NP, 0> eng{sH, sX, sT, sL, v.n, v.K, o.form, nullptr, nullptr, inst};
+    SimtEngine<NP, 0> eng{sH, sX, sT, sL, v.n, v.K, o.form, nullptr, nullptr, inst, &bl};
     solve_one<NP>(eng, v, o, slot, red, ctl);
     __syncthreads();
   }

@@ -208,7 +208,9 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
   const int K = a.K;
   if (K > kMaxK) return false;
   for (int e = tid; e < (1 + kMaxK + kMaxM) * 4; e += NT) (&ls.mask[0][0])[e] = 0u;
-  __syncthreads();
+  // the nonzeros of one row lie on as many diagonals: full matrices are told by one row
+  const float2 mid = tid < n ? __ldg(a.H + n / 2 * n + tid) : make_float2(0.f, 0.f);
+  if (__syncthreads_count(mid.x != 0.f || mid.y != 0.f) > kMaxH) return false;
   scan_diagonals<NT>(a.H, n, ls.mask[0]);
   for (int k = 0; k < K; ++k) scan_diagonals<NT>(a.L + (long long)k * n * n, n, ls.mask[1 + k]);
   for (int m = 0; m < M; ++m) scan_diagonals<NT>(td->ops + (long long)m * n * n, n, ls.mask[1 + kMaxK + m]);

@@ -390,6 +390,17 @@ __global__ void __launch_bounds__(32) band_kernel(Args a) {
     __syncwarp();
     if (lane < 8) mask[lane] = 0u;
     __syncwarp();
+    // the nonzeros of one row lie on as many diagonals: full matrices are told by one row
+    int mid = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float2 e = lane + 32 * r < n ? __ldg(H + (long long)(n / 2) * n + lane + 32 * r) : make_float2(0.f, 0.f);
+      mid += __popc(__ballot_sync(0xffffffffu, e.x != 0.f || e.y != 0.f));
+    }
+    if (mid > kMaxH) {
+      if (lane == 0) a.infos[inst * 3] = kPending;
+      continue;
+    }
     // nonzero diagonals (bit j - i + n - 1)
     constexpr int U = 8 / R;  // rows in flight
     for (int i0 = 0; i0 < n; i0 += U) {

@@ -55,10 +55,11 @@ def test_same_as_product_kernel(cuda_device, n, batch):  # two thread layouts up
 
 
 @pytest.mark.parametrize('jumps', [[], [(1, -1)], [(-2,), (0, 2)], [(-1,), (1,), (2,)]])
-@pytest.mark.parametrize('n', [13, 40])
+@pytest.mark.parametrize('n', [13, 32, 40, 64])
 def test_jump_patterns_and_options(cuda_device, n, jumps):
     H, Ls, rho, Es = _problem(n, 3, 3, jumps)
-    for kw in (dict(), dict(options=dq.Options(save_states=False)), dict(method=dq.Dopri5())):
+    for kw in (dict(), dict(options=dq.Options(save_states=False)), dict(method=dq.Dopri5()),
+               dict(options=dq.Options(assume_hermitian=False))):
         got = dq.mesolve(H, Ls, rho, [0.1, 0.1, 0.4], exp_ops=Es, **kw)
         ref = dq.mesolve(H + np.complex64(1e-25), Ls, rho, [0.1, 0.1, 0.4], exp_ops=Es, **kw)
         _agree(got, ref)
