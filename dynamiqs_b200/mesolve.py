@@ -30,6 +30,7 @@ from .method import Dopri5, Method, Tsit5
 from .options import Options, check_options
 from .qarrays import SparseDIA, to_dense
 from .result import AdaptiveStepInfos, MESolveResult
+from .upload import to_device
 
 __all__ = ['mesolve', 'MESolveB200Integrator']
 
@@ -234,14 +235,18 @@ def _device():
 
 
 def _to_dev(x, dtype, device):
+    return to_device({'x': (x, dtype)}, device)['x']
+
+
+def _stiffest_first(H, L, H_index, L_index):
+    """Instances sorted by a stiffness estimate, largest first (int32 tensor): the infinity
+    norm of Hnh = -iH - 1/2 sum L^+L bounded by ||H|| + 1/2 sum ||L||^2 (row sums)."""
     import torch
 
-    if isinstance(x, torch.Tensor):
-        return x.to(device=device, dtype=dtype).contiguous()
-    a = np.ascontiguousarray(x)
-    if not a.flags.writeable:  # a read-only view (e.g. a broadcast): torch wants its own copy
-        a = a.copy()
-    return torch.from_numpy(a).to(device=device, dtype=dtype).contiguous()
+    est = H.abs().sum(-1).amax(-1)[H_index.long()]
+    if L.shape[1]:
+        est = est + (0.5 * L.abs().sum(-1).amax(-1).square().sum(-1))[L_index.long()]
+    return torch.argsort(est, descending=True, stable=True).to(torch.int32)
 
 
 class PreparedSolve:
@@ -367,11 +372,19 @@ class MESolveB200Integrator:
                 else _lib.FORM_HERMITIAN)
 
     def run(self) -> MESolveResult:
-        return self.prepare().launch().result()
+        return self._prepare().launch().result()
 
     def prepare(self) -> PreparedSolve:
         """Copy the inputs to the device, size the workspace and bind the C-ABI call;
-        ``launch()`` may then be called repeatedly (the device inputs stay resident)."""
+        ``launch()`` may then be called repeatedly (the device inputs stay resident), on any
+        stream."""
+        import torch
+
+        prep = self._prepare()
+        torch.cuda.current_stream(prep.dev).synchronize()  # the copies, for other streams
+        return prep
+
+    def _prepare(self) -> PreparedSolve:
         lib = _lib.load()
         n = _shape(self.H)[-1]
         K = len(self.Ls)
@@ -414,13 +427,14 @@ class MESolveB200Integrator:
             if not herm.all():
                 raise RuntimeError('Argument y0 is not hermitian.')
         bufs = {
-            'superop_t': _to_dev(S_T, c64, dev),
-            'rho0': _to_dev(vectorize(rho)[..., 0], c64, dev),
-            'E': (_to_dev(np.stack([to_dense(E).reshape(-1) for E in self.Es]), c64, dev) if nE
-                  else torch.zeros(1, dtype=c64, device=dev)),
-            'tsave': _to_dev(np.asarray(self.ts, dtype=np.float64), torch.float64, dev),
-            'S_index': _to_dev(inverse.reshape(-1).astype(np.int32), torch.int32, dev),
-            'rho0_index': _to_dev(plan.rho_index, torch.int32, dev),
+            **to_device({
+                'superop_t': (S_T, c64),
+                'rho0': (vectorize(rho)[..., 0], c64),
+                'E': (np.stack([to_dense(E).reshape(-1) for E in self.Es]) if nE else np.zeros(1), c64),
+                'tsave': (self.ts, torch.float64),
+                'S_index': (inverse.reshape(-1), torch.int32),
+                'rho0_index': (plan.rho_index, torch.int32),
+            }, dev),
             'states': torch.empty((B, nsave, N), dtype=c64, device=dev),
             'expects': torch.empty((B, max(nE, 1), ntsave), dtype=c64, device=dev),
             'infos': torch.empty((B, 3), dtype=torch.int32, device=dev),
@@ -441,7 +455,8 @@ class MESolveB200Integrator:
 
         return PreparedSolve(self, fn, 'dqb_mesolve_vectorized', prob, outs, bufs, 256, dev, nE)
 
-    def _common_buffers(self, dev, n, ntsave, nE, B, nsave):
+    def _common_buffers(self, dev, n, ntsave, nE, B, nsave, operators):
+        """Device inputs (`operators`: the path's H and L arrays) and outputs of a solve."""
         import torch
 
         c64 = torch.complex64
@@ -449,13 +464,15 @@ class MESolveB200Integrator:
         r_items = plan.rho_items
         is_ket = r_items.shape[-1] == 1 and n > 1
         bufs = {
-            'rho0': _to_dev(r_items, c64, dev),
-            'E': (_to_dev(np.stack([to_dense(E) for E in self.Es]), c64, dev) if nE
-                  else torch.zeros(1, dtype=c64, device=dev)),
-            'tsave': _to_dev(np.asarray(self.ts, dtype=np.float64), torch.float64, dev),
-            'H_index': _to_dev(plan.H_index, torch.int32, dev),
-            'L_index': _to_dev(plan.L_index, torch.int32, dev),
-            'rho0_index': _to_dev(plan.rho_index, torch.int32, dev),
+            **to_device({
+                **{name: (x, c64) for name, x in operators.items()},
+                'rho0': (r_items, c64),
+                'E': (np.stack([to_dense(E) for E in self.Es]) if nE else np.zeros(1), c64),
+                'tsave': (self.ts, torch.float64),
+                'H_index': (plan.H_index, torch.int32),
+                'L_index': (plan.L_index, torch.int32),
+                'rho0_index': (plan.rho_index, torch.int32),
+            }, dev),
             'states': torch.empty((B, nsave, n, n), dtype=c64, device=dev),
             'expects': torch.empty((B, max(nE, 1), ntsave), dtype=c64, device=dev),
             'infos': torch.empty((B, 3), dtype=torch.int32, device=dev),
@@ -481,9 +498,8 @@ class MESolveB200Integrator:
         dev = _device()
         n, K, ntsave, B, nE, nsave = self._sizes()
         c64 = torch.complex64
-        bufs, outs, is_ket = self._common_buffers(dev, n, ntsave, nE, B, nsave)
-        bufs['H'] = _to_dev(self.plan.H_items_dense(), c64, dev)
-        bufs['L'] = _to_dev(self.plan.L_sets_dense(), c64, dev)
+        bufs, outs, is_ket = self._common_buffers(
+            dev, n, ntsave, nE, B, nsave, {'H': self.plan.H_items_dense(), 'L': self.plan.L_sets_dense()})
         prob = _lib.DenseProblem(
             n=n, n_jumps=K, n_exp=nE, n_tsave=ntsave, batch=B, H=bufs['H'].data_ptr(),
             L=bufs['L'].data_ptr(), rho0=bufs['rho0'].data_ptr(), rho0_is_ket=int(is_ket),
@@ -494,7 +510,8 @@ class MESolveB200Integrator:
             ws_bytes = lib.dqb_mesolve_dense_workspace_size(n, K + extra_mats, B)
             fn, name = lib.dqb_mesolve_dense, 'dqb_mesolve_dense'
             if B > 256:  # more instances than resident CTAs: start the stiffest first
-                bufs['start_order'] = _to_dev(self._start_order(), torch.int32, dev)
+                bufs['start_order'] = _stiffest_first(bufs['H'], bufs['L'], bufs['H_index'],
+                                                      bufs['L_index'])
                 prob.start_order = bufs['start_order'].data_ptr()
         else:
             ws_bytes = lib.dqb_mesolve_dense_large_workspace_size(n, K, nE, ntsave, B)
@@ -505,22 +522,15 @@ class MESolveB200Integrator:
         return PreparedSolve(self, fn, name, prob, outs, bufs, ws_bytes, dev, nE)
 
     def _start_order(self) -> np.ndarray:
-        """Instances sorted by a stiffness estimate, largest first: the infinity norm of
-        Hnh = -iH - 1/2 sum L^+L bounded by ||H|| + 1/2 sum ||L||^2 (row sums).  An
-        explicit RK step size scales roughly with the inverse of that spectral radius, so
-        this starts the longest solves first and leaves short ones for the tail of the
-        persistent kernel.  Changes only the order of work, not any result."""
+        """The start order of the instances, as ``_prepare_dense`` forms it on the device: an
+        explicit RK step size scales roughly with the inverse of the spectral radius, so
+        stiffest first starts the longest solves first and leaves short ones for the tail of
+        the persistent kernel.  Changes only the order of work, not any result."""
+        import torch
+
         plan = self.plan
-        H = plan.H_items_dense()
-        h = np.abs(H).sum(-1).max(-1)
-        Ls = plan.L_sets_dense()
-        if Ls.shape[1]:
-            lnorm = np.abs(Ls).sum(-1).max(-1)
-            l_est = 0.5 * (lnorm ** 2).sum(-1)
-        else:
-            l_est = np.zeros(Ls.shape[0])
-        est = h[np.asarray(plan.H_index)] + l_est[np.asarray(plan.L_index)]
-        return np.argsort(-est, kind='stable').astype(np.int32)
+        return _stiffest_first(*(torch.from_numpy(np.array(x)) for x in (
+            plan.H_items_dense(), plan.L_sets_dense(), plan.H_index, plan.L_index))).numpy()
 
     def _tune_gemm_precision(self, lib, prob, ws, ws_bytes, dev) -> None:
         """``precision='auto'``: the faster of FP32 and 3xTF32 products for this (n, K,
@@ -565,13 +575,12 @@ class MESolveB200Integrator:
         n, K, ntsave, B, nE, nsave = self._sizes()
         plan = self.plan
         c64 = torch.complex64
-        bufs, outs, is_ket = self._common_buffers(dev, n, ntsave, nE, B, nsave)
         H = plan.H_items if isinstance(plan.H_items, SparseDIA) else SparseDIA.from_dense(plan.H_items)
         Lsets = plan.L_sets if isinstance(plan.L_sets, list) else [
             SparseDIA.from_dense(plan.L_sets[:, k]) for k in range(plan.L_sets.shape[1])]
-        bufs['H'] = _to_dev(H.diags, c64, dev)
-        bufs['L'] = (_to_dev(np.concatenate([L.diags for L in Lsets], axis=-2), c64, dev)
-                     if Lsets else torch.zeros(1, dtype=c64, device=dev))
+        bufs, outs, is_ket = self._common_buffers(
+            dev, n, ntsave, nE, B, nsave,
+            {'H': H.diags, 'L': (np.concatenate([L.diags for L in Lsets], axis=-2) if Lsets else np.zeros(1))})
         l_off_list = [k for L in Lsets for k in L.offsets]
         host = {  # host arrays the C ABI reads during the call
             'h_off': (ctypes.c_int32 * max(len(H.offsets), 1))(*H.offsets),
@@ -667,12 +676,12 @@ class MESolveB200Integrator:
     def _result(self, states, expects, infos, status) -> MESolveResult:
         import torch
 
-        st = status.cpu()
-        if bool((st == _lib.INST_NOT_HERMITIAN).any()):
+        st = status.cpu().numpy()
+        if (st == _lib.INST_NOT_HERMITIAN).any():
             raise RuntimeError('Argument y0 is not hermitian.')
-        if bool((st == _lib.INST_MAX_STEPS).any()):
+        if (st == _lib.INST_MAX_STEPS).any():
             raise RuntimeError(_MAX_STEPS_MSG)
-        if bool((st == _lib.INST_NONFINITE).any()):
+        if (st == _lib.INST_NONFINITE).any():
             raise RuntimeError('The solution became non-finite (NaN or inf) during the '
                                'integration.')
         bshape = self.plan.bshape
@@ -835,8 +844,6 @@ def _mesolve_td(Hs, jump_ops, rho0, tsave, *, exp_ops, method, gradient, options
 
     import torch
 
-    from .time_qarray import PWCTimeQArray
-
     Ls = [_as_op(_jump_source(L)) for L in jump_ops]
     rho0 = _as_op(rho0)
     tsave = np.asarray(tsave.detach().cpu().numpy() if hasattr(tsave, 'detach') else tsave,
@@ -867,34 +874,13 @@ def _mesolve_td(Hs, jump_ops, rho0, tsave, *, exp_ops, method, gradient, options
         prep.bufs['workspace'] = torch.empty(max(wsb, 1), dtype=torch.uint8, device=prep.dev)
         prep.ws_bytes = wsb
     dev = prep.dev
-    nsets = int(np.prod(bs, dtype=np.int64)) if bs else 1
-    terms = (_lib.TdTerm * _lib.TD_MAX_TERMS)()
-    keep = []
-    for m, term in enumerate(Hs.td_terms):
-        T = terms[m]
-        if isinstance(term, PWCTimeQArray):
-            vals = np.broadcast_to(term.values, (*bs, term.values.shape[-1])).reshape(nsets, -1)
-            tt = _to_dev(term.times, torch.float64, dev)
-            vv = _to_dev(np.ascontiguousarray(vals, dtype=np.complex128), torch.complex128, dev)
-            keep += [tt, vv]
-            T.kind, T.n_times = _lib.TD_PWC, term.times.size
-            T.times, T.values = tt.data_ptr(), vv.data_ptr()
-            T.value_index = prep.bufs['H_index'].data_ptr() if bs else None
-        else:
-            f = term.f
-            T.kind = _lib.TD_WAVE
-            T.amp_re, T.amp_im = f.amplitude.real, f.amplitude.imag
-            T.omega, T.phase, T.t_center, T.sigma = f.omega, f.phase, f.t_center, f.sigma
-            T.t_start, T.t_end = f.t_start, f.t_end
-    ops_d = (_to_dev(np.stack([t.qarray for t in Hs.td_terms]), torch.complex64, dev)
-             if Hs.td_terms else torch.zeros(1, dtype=torch.complex64, device=dev))
-    jterms, disc = _jump_prefactors(jump_ops, dev, keep)
-    jts = np.unique(np.concatenate([np.asarray(Hs.discontinuity_ts, dtype=np.float64)] + disc))
-    jts_d = _to_dev(jts if jts.size else np.zeros(1), torch.float64, dev)
-    keep += [ops_d, jts_d]
+    jterms, disc, keep = _jump_prefactors(jump_ops, dev)
+    terms, ops_d, jts_d, n_jts, up = _td_device(
+        Hs, bs, [t.qarray for t in Hs.td_terms], disc, prep.bufs['H_index'] if bs else None, dev)
+    keep.append(up)
     td = _lib.TdHamiltonian(n_terms=len(Hs.td_terms), ops=ops_d.data_ptr(),
                             terms=ctypes.cast(terms, ctypes.POINTER(_lib.TdTerm)),
-                            n_jump_ts=int(jts.size), jump_ts=jts_d.data_ptr(),
+                            n_jump_ts=n_jts, jump_ts=jts_d.data_ptr(),
                             jump_terms=(ctypes.cast(jterms, ctypes.POINTER(_lib.TdTerm))
                                         if jterms is not None else None))
     prep.bufs['td'] = (td, terms, keep)
@@ -919,15 +905,52 @@ def _td_on_dia(Hs, jump_ops, options) -> bool:
     return len(_td_union_offsets(Hs)) <= _lib.DIA_MAX_HNH_DIAGS
 
 
-def _jump_prefactors(jump_ops, dev, keep):
+def _td_device(Hs, bs, ops, disc, value_index, dev):
+    """Device side of a time-dependent H: the dqb_td_term array of its prefactors (batched PWC
+    values ``(*bs, N)`` indexed by ``value_index``), its operators ``ops`` and the sorted
+    discontinuity times (H's and the lists in ``disc``) with their number, in one upload, which
+    the caller keeps alive."""
+    import torch
+
+    from .time_qarray import PWCTimeQArray
+
+    nsets = int(np.prod(bs, dtype=np.int64)) if bs else 1
+    jts = np.unique(np.concatenate([np.asarray(Hs.discontinuity_ts, dtype=np.float64)] + disc))
+    items = {'ops': (np.stack(ops) if ops else np.zeros(1), torch.complex64),
+             'jump_ts': (jts if jts.size else np.zeros(1), torch.float64)}
+    for m, term in enumerate(Hs.td_terms):
+        if isinstance(term, PWCTimeQArray):
+            vals = np.broadcast_to(term.values, (*bs, term.values.shape[-1])).reshape(nsets, -1)
+            items[f'times{m}'] = (term.times, torch.float64)
+            items[f'values{m}'] = (vals, torch.complex128)
+    up = to_device(items, dev)
+    terms = (_lib.TdTerm * _lib.TD_MAX_TERMS)()
+    for m, term in enumerate(Hs.td_terms):
+        T = terms[m]
+        if isinstance(term, PWCTimeQArray):
+            T.kind, T.n_times = _lib.TD_PWC, term.times.size
+            T.times, T.values = up[f'times{m}'].data_ptr(), up[f'values{m}'].data_ptr()
+            T.value_index = value_index.data_ptr() if value_index is not None else None
+        else:
+            f = term.f
+            T.kind = _lib.TD_WAVE
+            T.amp_re, T.amp_im = f.amplitude.real, f.amplitude.imag
+            T.omega, T.phase, T.t_center, T.sigma = f.omega, f.phase, f.t_center, f.sigma
+            T.t_start, T.t_end = f.t_start, f.t_end
+    return terms, up['ops'], up['jump_ts'], int(jts.size), up
+
+
+def _jump_prefactors(jump_ops, dev):
     """The dqb_td_term array of the jump operators' prefactors c_k(t) (constant operators:
-    DQB_TD_CONST), or None when none depends on time, and their discontinuity times."""
+    DQB_TD_CONST), or None when none depends on time, their discontinuity times, and what the
+    caller keeps alive."""
     import torch
 
     from .time_qarray import ModulatedTimeQArray, PWCTimeQArray
 
+    keep = []
     if not any(isinstance(L, (PWCTimeQArray, ModulatedTimeQArray)) for L in jump_ops):
-        return None, []
+        return None, [], keep
     jterms = (_lib.TdTerm * max(len(jump_ops), 1))()
     disc = []
     for k, L in enumerate(jump_ops):
@@ -950,7 +973,7 @@ def _jump_prefactors(jump_ops, dev, keep):
         else:
             T.kind = _lib.TD_CONST
     keep.append(jterms)
-    return jterms, disc
+    return jterms, disc, keep
 
 
 def _td_jumps_on_large(Hs, jump_ops, options) -> bool:
@@ -1003,10 +1026,6 @@ def _mesolve_td_dia(Hs, jump_ops, rho0, tsave, *, exp_ops, method, gradient, opt
     result dimensions (cartesian batching), as on the n <= 64 kernel."""
     import ctypes
 
-    import torch
-
-    from .time_qarray import PWCTimeQArray
-
     Ls = [_jump_source(L) for L in jump_ops]
     rho0 = _as_op(rho0)
     tsave = np.asarray(tsave.detach().cpu().numpy() if hasattr(tsave, 'detach') else tsave,
@@ -1035,35 +1054,14 @@ def _mesolve_td_dia(Hs, jump_ops, rho0, tsave, *, exp_ops, method, gradient, opt
     lib = _lib.load()
     prep = integ._prepare_dia(lib)
     dev = prep.dev
-    nsets = int(np.prod(bs, dtype=np.int64)) if bs else 1
-    terms = (_lib.TdTerm * _lib.TD_MAX_TERMS)()
-    keep = []
-    for m, term in enumerate(Hs.td_terms):
-        T = terms[m]
-        if isinstance(term, PWCTimeQArray):
-            vals = np.broadcast_to(term.values, (*bs, term.values.shape[-1])).reshape(nsets, -1)
-            tt = _to_dev(term.times, torch.float64, dev)
-            vv = _to_dev(np.ascontiguousarray(vals, dtype=np.complex128), torch.complex128, dev)
-            keep += [tt, vv]
-            T.kind, T.n_times = _lib.TD_PWC, term.times.size
-            T.times, T.values = tt.data_ptr(), vv.data_ptr()
-            T.value_index = prep.bufs['H_index'].data_ptr() if bs else None
-        else:
-            f = term.f
-            T.kind = _lib.TD_WAVE
-            T.amp_re, T.amp_im = f.amplitude.real, f.amplitude.imag
-            T.omega, T.phase, T.t_center, T.sigma = f.omega, f.phase, f.t_center, f.sigma
-            T.t_start, T.t_end = f.t_start, f.t_end
-    ops_d = (_to_dev(np.stack([_on_offsets(t.source, offs) for t in Hs.td_terms]), torch.complex64, dev)
-             if Hs.td_terms else torch.zeros(1, dtype=torch.complex64, device=dev))
-    # prefactors of the jump operators (constant ones: 1)
-    jterms, disc = _jump_prefactors(jump_ops, dev, keep)
-    jts = np.unique(np.concatenate([np.asarray(Hs.discontinuity_ts, dtype=np.float64)] + disc))
-    jts_d = _to_dev(jts if jts.size else np.zeros(1), torch.float64, dev)
-    keep += [ops_d, jts_d]
+    jterms, disc, keep = _jump_prefactors(jump_ops, dev)
+    terms, ops_d, jts_d, n_jts, up = _td_device(
+        Hs, bs, [_on_offsets(t.source, offs) for t in Hs.td_terms], disc,
+        prep.bufs['H_index'] if bs else None, dev)
+    keep.append(up)
     td = _lib.TdHamiltonian(n_terms=len(Hs.td_terms), ops=ops_d.data_ptr(),
                             terms=ctypes.cast(terms, ctypes.POINTER(_lib.TdTerm)),
-                            n_jump_ts=int(jts.size), jump_ts=jts_d.data_ptr(),
+                            n_jump_ts=n_jts, jump_ts=jts_d.data_ptr(),
                             jump_terms=(ctypes.cast(jterms, ctypes.POINTER(_lib.TdTerm))
                                         if jterms is not None else None))
     prep.bufs['td'] = (td, terms, jterms, keep)

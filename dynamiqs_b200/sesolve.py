@@ -20,12 +20,13 @@ from dataclasses import dataclass
 import numpy as np
 
 from . import _lib
-from .mesolve import (_as_op, _check_shape, _device, _MAX_STEPS_MSG, _shape, _to_dev,
+from .mesolve import (_as_op, _check_shape, _device, _MAX_STEPS_MSG, _shape,
                       assert_method_supported, check_times, make_batch_plan)
 from .method import Method, Tsit5
 from .options import Options, check_options
 from .qarrays import SparseDIA, to_dense
 from .result import AdaptiveStepInfos, MESolveResult
+from .upload import to_device
 
 __all__ = ['sesolve', 'SESolveResult', 'SESolveB200Integrator']
 
@@ -121,6 +122,13 @@ class SESolveB200Integrator:
         return 'dia' if isinstance(self.plan.H_items, SparseDIA) else 'dense_large'
 
     def prepare(self) -> _Prepared:
+        import torch
+
+        prep = self._prepare()
+        torch.cuda.current_stream().synchronize()  # the copies, for launches on other streams
+        return prep
+
+    def _prepare(self) -> _Prepared:
         import ctypes
 
         import torch
@@ -146,13 +154,14 @@ class SESolveB200Integrator:
         if ws_bytes == 0:
             raise NotImplementedError(f'sesolve on the B200 path supports n <= {LARGE_MAX_N}.')
         bufs = {
-            'H': _to_dev(plan.H_items.diags if dia else plan.H_items_dense(), c64, dev),
-            'psi0': _to_dev(plan.rho_items, c64, dev),
-            'E': (_to_dev(np.stack([to_dense(E) for E in self.Es]), c64, dev) if nE
-                  else torch.zeros(1, dtype=c64, device=dev)),
-            'tsave': _to_dev(np.asarray(self.ts, dtype=np.float64), torch.float64, dev),
-            'H_index': _to_dev(plan.H_index, torch.int32, dev),
-            'psi0_index': _to_dev(plan.rho_index, torch.int32, dev),
+            **to_device({
+                'H': (plan.H_items.diags if dia else plan.H_items_dense(), c64),
+                'psi0': (plan.rho_items, c64),
+                'E': (np.stack([to_dense(E) for E in self.Es]) if nE else np.zeros(1), c64),
+                'tsave': (self.ts, torch.float64),
+                'H_index': (plan.H_index, torch.int32),
+                'psi0_index': (plan.rho_index, torch.int32),
+            }, dev),
             'states': torch.empty((B, nsave, n, 1), dtype=c64, device=dev),
             'expects': torch.empty((B, max(nE, 1), ntsave), dtype=c64, device=dev),
             'infos': torch.empty((B, 3), dtype=torch.int32, device=dev),
@@ -190,13 +199,13 @@ class SESolveB200Integrator:
         return _Prepared(self, prob, outs, bufs, fn, host, td)
 
     def run(self) -> SESolveResult:
-        return self.prepare().launch().result()
+        return self._prepare().launch().result()
 
     def _result(self, b) -> SESolveResult:
-        st = b['status'].cpu()
-        if bool((st == _lib.INST_MAX_STEPS).any()):
+        st = b['status'].cpu().numpy()
+        if (st == _lib.INST_MAX_STEPS).any():
             raise RuntimeError(_MAX_STEPS_MSG)
-        if bool((st == _lib.INST_NONFINITE).any()):
+        if (st == _lib.INST_NONFINITE).any():
             raise RuntimeError('The solution became non-finite (NaN or inf) during the '
                                'integration.')
         bshape = self.plan.bshape
@@ -235,43 +244,16 @@ def _td_struct(Hs, plan, bufs, dev, dia):
     part (dense, or diagonals on its offsets)."""
     import ctypes
 
-    import torch
-
-    from .mesolve import _on_offsets
-    from .time_qarray import PWCTimeQArray
+    from .mesolve import _on_offsets, _td_device
 
     bs = tuple(Hs.batch_shape)
-    nsets = int(np.prod(bs, dtype=np.int64)) if bs else 1
-    terms = (_lib.TdTerm * _lib.TD_MAX_TERMS)()
-    keep = []
-    for m, term in enumerate(Hs.td_terms):
-        T = terms[m]
-        if isinstance(term, PWCTimeQArray):
-            vals = np.broadcast_to(term.values, (*bs, term.values.shape[-1])).reshape(nsets, -1)
-            tt = _to_dev(term.times, torch.float64, dev)
-            vv = _to_dev(np.ascontiguousarray(vals, dtype=np.complex128), torch.complex128, dev)
-            keep += [tt, vv]
-            T.kind, T.n_times = _lib.TD_PWC, term.times.size
-            T.times, T.values = tt.data_ptr(), vv.data_ptr()
-            T.value_index = bufs['H_index'].data_ptr() if bs else None
-        else:
-            f = term.f
-            T.kind = _lib.TD_WAVE
-            T.amp_re, T.amp_im = f.amplitude.real, f.amplitude.imag
-            T.omega, T.phase, T.t_center, T.sigma = f.omega, f.phase, f.t_center, f.sigma
-            T.t_start, T.t_end = f.t_start, f.t_end
-    if dia:
-        offs = tuple(plan.H_items.offsets)
-        ops = np.stack([_on_offsets(t.source, offs) for t in Hs.td_terms])
-    else:
-        ops = np.stack([t.qarray for t in Hs.td_terms])
-    ops_d = _to_dev(ops, torch.complex64, dev)
-    jts = np.asarray(Hs.discontinuity_ts, dtype=np.float64)
-    jts_d = _to_dev(jts if jts.size else np.zeros(1), torch.float64, dev)
-    keep += [ops_d, jts_d, terms]
+    offs = tuple(plan.H_items.offsets) if dia else ()
+    ops = [_on_offsets(t.source, offs) if dia else t.qarray for t in Hs.td_terms]
+    terms, ops_d, jts_d, n_jts, up = _td_device(Hs, bs, ops, [], bufs['H_index'] if bs else None, dev)
+    keep = [up, terms]
     td = _lib.TdHamiltonian(n_terms=len(Hs.td_terms), ops=ops_d.data_ptr(),
                             terms=ctypes.cast(terms, ctypes.POINTER(_lib.TdTerm)),
-                            n_jump_ts=int(jts.size), jump_ts=jts_d.data_ptr())
+                            n_jump_ts=n_jts, jump_ts=jts_d.data_ptr())
     return td, keep
 
 

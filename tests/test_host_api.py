@@ -210,3 +210,27 @@ def test_time_dependent_jump_operators_need_one_storage():
     with pytest.raises(NotImplementedError, match='unbatched values'):
         dq.mesolve(ops.dag(a) @ a, [dq.pwc([0.0, 1.0], [[1.0], [0.5]], a)], ops.fock(6, 0),
                    [0.0, 1.0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('nbytes', [0, 8, 1 << 18, (1 << 18) + 8, 8 << 20, (24 << 20) - 8, 24 << 20, (57 << 20) + 24])
+def test_upload_is_the_array(cuda_device, nbytes):
+    """Packed, slot-sized and ring-wrapping arrays, read-only and converted ones, in one upload
+    and again with new contents straight after."""
+    import torch
+
+    from dynamiqs_b200.upload import to_device
+
+    rng = np.random.default_rng(nbytes)
+    for _ in range(2):
+        a = rng.normal(size=nbytes // 8).astype(np.float32).view(np.float32)
+        a = (a + 1j * a[::-1]).astype(np.complex64).reshape(-1)
+        ro = np.broadcast_to(np.float64(2.5), (3, 5))
+        idx = np.arange(7)
+        out = to_device({'a': (a, torch.complex64), 'ro': (ro, torch.complex64), 'i': (idx, torch.int32)},
+                        torch.device('cuda', 0))
+        want = a.copy()
+        a[:] = 0
+        assert np.array_equal(out['a'].cpu().numpy(), want)
+        assert np.array_equal(out['ro'].cpu().numpy(), ro.astype(np.complex64))
+        assert out['i'].dtype == torch.int32 and out['i'].tolist() == list(range(7))
