@@ -276,9 +276,9 @@ SIGNATURES = {
                                           ctypes.c_size_t, _P]),
     'dqb_mesolve_vectorized': (ctypes.c_int, [ctypes.POINTER(DenseProblem), _P, ctypes.POINTER(OdeOptions),
                                               ctypes.POINTER(Outputs), _P, ctypes.c_size_t, _P]),
-    'dqb_state_hermiticity_workspace_size': (ctypes.c_size_t, [ctypes.c_int32, ctypes.c_int64]),
-    'dqb_state_hermiticity': (ctypes.c_int, [_P, ctypes.c_int32, ctypes.c_int64, _P, _P,
-                                             ctypes.c_size_t, _P]),
+    'dqb_state_checks_workspace_size': (ctypes.c_size_t, [ctypes.c_int32, ctypes.c_int64]),
+    'dqb_state_checks': (ctypes.c_int, [_P, ctypes.c_int32, ctypes.c_int64, _P, _P, _P,
+                                        ctypes.c_size_t, _P]),
     'dqb_version': (ctypes.c_char_p, []),
 }
 

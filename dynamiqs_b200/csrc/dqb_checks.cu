@@ -1,4 +1,4 @@
-// Hermiticity defect ||rho - rho^+||_F / ||rho||_F of saved states, in FP64.
+// Hermiticity defect ||rho - rho^+||_F / ||rho||_F and trace of saved states, in FP64.
 //
 // Bound: HBM, every state read once (the FP64 conversions, 16 per SM and cycle, come next).
 // A block takes the tile pair (ti, tj), (tj, ti) of 32 x 32 tiles, ti <= tj, reads both row
@@ -21,17 +21,21 @@ namespace {
 
 constexpr int kCT = 32;
 
-// blockIdx.x = state * blocks + part; partial[blockIdx.x] = (sum |rho - rho^+|^2, sum |rho|^2)
-// over the part's tile pairs.
-__global__ void __launch_bounds__(256) herm_partial_kernel(const float2* __restrict__ states, int n, int blocks,
-                                                           double2* __restrict__ partial) {
+struct Partial {
+  double num, den;     // sum |rho - rho^+|^2, sum |rho|^2
+  double tr_re, tr_im;  // sum rho_ii
+};
+
+// blockIdx.x = state * blocks + part; partial[blockIdx.x]: the sums over the part's tile pairs.
+__global__ void __launch_bounds__(256) checks_partial_kernel(const float2* __restrict__ states, int n, int blocks,
+                                                             Partial* __restrict__ partial) {
   __shared__ float2 sh[kCT][kCT + 1];
   __shared__ double red[72];
   const long long s = blockIdx.x / blocks;
   const float2* __restrict__ M = states + s * n * n;
   const int T = (n + kCT - 1) / kCT, pairs = T * (T + 1) / 2;
   const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
-  double num = 0.0, den = 0.0;
+  double num = 0.0, den = 0.0, tr = 0.0, ti_sum = 0.0;
   int p = (int)(blockIdx.x % blocks), ti = 0, at = 0;  // row ti of the pairs starts at `at`
   for (; p < pairs; p += blocks) {
     while (p - at >= T - ti) at += T - ti, ++ti;
@@ -54,26 +58,30 @@ __global__ void __launch_bounds__(256) herm_partial_kernel(const float2* __restr
         num += w * (dx * dx + dy * dy);
         den += ax * ax + ay * ay;
         if (ti != tj) den += bx * bx + by * by;
+        if (r == c) tr += ax, ti_sum += ay;
       }
     }
   }
-  const double2 v = block_sum2(num, den, red);
-  if (threadIdx.x == 0) partial[blockIdx.x] = v;
+  const double2 v = block_sum2(num, den, red), t = block_sum2(tr, ti_sum, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = Partial{v.x, v.y, t.x, t.y};
 }
 
 // One thread per state.
-__global__ void herm_ratio_kernel(const double2* __restrict__ partial, long long count, int blocks,
-                                  double* __restrict__ out) {
+__global__ void checks_sum_kernel(const Partial* __restrict__ partial, long long count, int blocks,
+                                  double* __restrict__ herm, double2* __restrict__ trace) {
   const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (s >= count) return;
-  double num = 0.0, den = 0.0;
+  Partial v{0.0, 0.0, 0.0, 0.0};
   for (int b = 0; b < blocks; ++b) {
-    const double2 v = partial[s * blocks + b];
-    num += v.x;
-    den += v.y;
+    const Partial p = partial[s * blocks + b];
+    v.num += p.num;
+    v.den += p.den;
+    v.tr_re += p.tr_re;
+    v.tr_im += p.tr_im;
   }
-  den = sqrt(den);
-  out[s] = sqrt(num) / (den < 1e-300 ? 1e-300 : den);
+  const double den = sqrt(v.den);
+  herm[s] = sqrt(v.num) / (den < 1e-300 ? 1e-300 : den);
+  trace[s] = make_double2(v.tr_re, v.tr_im);
 }
 
 // Blocks per state: eight per SM over all states, at most one per tile pair.
@@ -85,23 +93,23 @@ int blocks_per_state(int n, long long count) {
 }  // namespace
 }  // namespace dqb
 
-extern "C" size_t dqb_state_hermiticity_workspace_size(int32_t n, int64_t count) {
+extern "C" size_t dqb_state_checks_workspace_size(int32_t n, int64_t count) {
   if (n < 1 || count < 1) return 0;
-  return (size_t)count * dqb::blocks_per_state(n, count) * sizeof(double2);
+  return (size_t)count * dqb::blocks_per_state(n, count) * sizeof(dqb::Partial);
 }
 
-extern "C" int dqb_state_hermiticity(const void* states, int32_t n, int64_t count, double* out, void* workspace,
-                                     size_t workspace_bytes, void* stream) {
+extern "C" int dqb_state_checks(const void* states, int32_t n, int64_t count, double* hermiticity, void* trace,
+                                void* workspace, size_t workspace_bytes, void* stream) {
   if (n < 1 || count < 0) return DQB_ERR_INVALID_ARGUMENT;
   if (count == 0) return DQB_OK;
-  if (!states || !out) return DQB_ERR_INVALID_ARGUMENT;
+  if (!states || !hermiticity || !trace) return DQB_ERR_INVALID_ARGUMENT;
   const int blocks = dqb::blocks_per_state(n, count);
   if (count > (int64_t)0x7fffffff / blocks) return DQB_ERR_UNSUPPORTED;
-  if (!workspace || workspace_bytes < dqb_state_hermiticity_workspace_size(n, count))
-    return DQB_ERR_WORKSPACE_TOO_SMALL;
+  if (!workspace || workspace_bytes < dqb_state_checks_workspace_size(n, count)) return DQB_ERR_WORKSPACE_TOO_SMALL;
   cudaStream_t s = (cudaStream_t)stream;
-  double2* partial = (double2*)workspace;
-  dqb::herm_partial_kernel<<<(unsigned)(count * blocks), 256, 0, s>>>((const float2*)states, n, blocks, partial);
-  dqb::herm_ratio_kernel<<<(unsigned)((count + 127) / 128), 128, 0, s>>>(partial, count, blocks, out);
+  dqb::Partial* partial = (dqb::Partial*)workspace;
+  dqb::checks_partial_kernel<<<(unsigned)(count * blocks), 256, 0, s>>>((const float2*)states, n, blocks, partial);
+  dqb::checks_sum_kernel<<<(unsigned)((count + 127) / 128), 128, 0, s>>>(partial, count, blocks, hermiticity,
+                                                                        (double2*)trace);
   return cudaGetLastError() == cudaSuccess ? DQB_OK : DQB_ERR_CUDA;
 }

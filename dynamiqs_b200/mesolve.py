@@ -238,6 +238,13 @@ def _to_dev(x, dtype, device):
     return to_device({'x': (x, dtype)}, device)['x']
 
 
+def _stacked(Es):
+    """Expectation operators as one array (a view of a single one)."""
+    if len(Es) == 1:
+        return to_dense(Es[0])[None]
+    return np.stack([to_dense(E) for E in Es]) if Es else np.zeros(1)
+
+
 def _stiffest_first(H, L, H_index, L_index):
     """Instances sorted by a stiffness estimate, largest first (int32 tensor): the infinity
     norm of Hnh = -iH - 1/2 sum L^+L bounded by ||H|| + 1/2 sum ||L||^2 (row sums)."""
@@ -340,10 +347,13 @@ class MESolveB200Integrator:
         self.options = options
         self.H = H
         self.Ls = Ls
-        # The identity is appended to the expectation operators: its FP64-summed expectation
-        # value at every save point is the trace check of the saved states (result.checks).
+        # The trace check (result.checks) comes from the saved states.  Where only the final
+        # state is kept the identity is one more expectation operator, whose FP64-summed
+        # expectation value is the trace at every save point.
         self._n_user_E = len(Es) if Es else 0
-        self.Es = list(Es or []) + [np.eye(_shape(H)[-1], dtype=np.complex64)]
+        self.Es = list(Es or [])
+        if not options.save_states:
+            self.Es.append(np.eye(_shape(H)[-1], dtype=np.complex64))
         self.plan = plan
         self._tuned: dict = {}  # launch choices made by the autotuner at prepare time
         self._path = 'large'  # 'small', 'large' or 'dia': set by prepare()
@@ -467,7 +477,7 @@ class MESolveB200Integrator:
             **to_device({
                 **{name: (x, c64) for name, x in operators.items()},
                 'rho0': (r_items, c64),
-                'E': (np.stack([to_dense(E) for E in self.Es]) if nE else np.zeros(1), c64),
+                'E': (_stacked(self.Es), c64),
                 'tsave': (self.ts, torch.float64),
                 'H_index': (plan.H_index, torch.int32),
                 'L_index': (plan.L_index, torch.int32),
@@ -650,9 +660,9 @@ class MESolveB200Integrator:
         return self._prepare_dia(lib).launch().result()
 
     def _checks(self, states, trace):
-        """FP64 checks of the saved states: tr(rho) at every save point (the identity's
-        expectation value, summed in FP64 by the kernels) and the hermiticity defect
-        ||rho - rho^+||_F / ||rho||_F of every saved state (FP64, on the device)."""
+        """FP64 checks of the saved states: tr(rho) at every save point (``trace`` where only the
+        final state is kept) and the hermiticity defect ||rho - rho^+||_F / ||rho||_F of every
+        saved state (FP64, on the device)."""
         import torch
 
         n = states.shape[-1]
@@ -660,18 +670,22 @@ class MESolveB200Integrator:
             st = states.to(torch.complex128)
             den = torch.linalg.norm(st.reshape(*st.shape[:-2], -1), dim=-1)
             num = torch.linalg.norm((st - st.mH).reshape(*st.shape[:-2], -1), dim=-1)
-            return {'trace': trace, 'hermiticity': num / torch.clamp(den, min=1e-300)}
-        # (a transposed view, as the vectorized form returns, has the same defect)
-        st = states if states.is_contiguous() else states.transpose(-1, -2).contiguous()
-        count = states.numel() // (n * n)
-        lib = _lib.load()
-        out = torch.empty(states.shape[:-2], dtype=torch.float64, device=states.device)
-        size = lib.dqb_state_hermiticity_workspace_size(n, count)
-        ws = torch.empty(size, dtype=torch.uint8, device=states.device)
-        rc = lib.dqb_state_hermiticity(st.data_ptr(), n, count, out.data_ptr(), ws.data_ptr(), size,
-                                       torch.cuda.current_stream(states.device).cuda_stream)
-        _lib.check(rc, 'dqb_state_hermiticity')
-        return {'trace': trace, 'hermiticity': out}
+            herm = num / torch.clamp(den, min=1e-300)
+            tr = st.diagonal(dim1=-2, dim2=-1).sum(-1)
+        else:
+            # (a transposed view, as the vectorized form returns, has the same defect and trace)
+            st = states if states.is_contiguous() else states.transpose(-1, -2).contiguous()
+            count = states.numel() // (n * n)
+            lib = _lib.load()
+            herm = torch.empty(states.shape[:-2], dtype=torch.float64, device=states.device)
+            tr = torch.empty(states.shape[:-2], dtype=torch.complex128, device=states.device)
+            size = lib.dqb_state_checks_workspace_size(n, count)
+            ws = torch.empty(size, dtype=torch.uint8, device=states.device)
+            rc = lib.dqb_state_checks(st.data_ptr(), n, count, herm.data_ptr(), tr.data_ptr(),
+                                      ws.data_ptr(), size,
+                                      torch.cuda.current_stream(states.device).cuda_stream)
+            _lib.check(rc, 'dqb_state_checks')
+        return {'trace': tr if trace is None else trace, 'hermiticity': herm}
 
     def _result(self, states, expects, infos, status) -> MESolveResult:
         import torch
@@ -686,9 +700,10 @@ class MESolveB200Integrator:
                                'integration.')
         bshape = self.plan.bshape
         trace = None
-        if expects is not None:  # the last row is the identity's: the trace check
+        if expects is not None and not self.options.save_states:  # the identity's row
             trace = expects[:, self._n_user_E].to(torch.complex128)
             trace = trace.reshape(*bshape, trace.shape[-1])
+        if expects is not None:
             expects = expects[:, :self._n_user_E] if self._n_user_E else None
         if self._path == 'vectorized':  # vec(rho) -> rho (unvectorize, columns stacked)
             m = int(round(states.shape[-1] ** 0.5))

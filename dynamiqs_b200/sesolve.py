@@ -20,7 +20,7 @@ from dataclasses import dataclass
 import numpy as np
 
 from . import _lib
-from .mesolve import (_as_op, _check_shape, _device, _MAX_STEPS_MSG, _shape,
+from .mesolve import (_as_op, _check_shape, _device, _MAX_STEPS_MSG, _shape, _stacked,
                       assert_method_supported, check_times, make_batch_plan)
 from .method import Method, Tsit5
 from .options import Options, check_options
@@ -157,7 +157,7 @@ class SESolveB200Integrator:
             **to_device({
                 'H': (plan.H_items.diags if dia else plan.H_items_dense(), c64),
                 'psi0': (plan.rho_items, c64),
-                'E': (np.stack([to_dense(E) for E in self.Es]) if nE else np.zeros(1), c64),
+                'E': (_stacked(self.Es), c64),
                 'tsave': (self.ts, torch.float64),
                 'H_index': (plan.H_index, torch.int32),
                 'psi0_index': (plan.rho_index, torch.int32),

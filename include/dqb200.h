@@ -560,13 +560,14 @@ DQB_API int dqb_lindblad_rhs_dia_tiled(const dqb_dia_problem* problem, int32_t f
                                        size_t workspace_bytes, void* stream);
 
 /* ---- checks of saved states ----------------------------------------------------- */
-/* Scratch bytes of dqb_state_hermiticity. */
-DQB_API size_t dqb_state_hermiticity_workspace_size(int32_t n, int64_t count);
+/* Scratch bytes of dqb_state_checks. */
+DQB_API size_t dqb_state_checks_workspace_size(int32_t n, int64_t count);
 
-/* Hermiticity defect ||rho - rho^+||_F / ||rho||_F of `count` states (complex64 [count, n, n],
- * device) into out (float64 [count], device), FP64 sums; a zero state gives 0. */
-DQB_API int dqb_state_hermiticity(const void* states, int32_t n, int64_t count, double* out,
-                                  void* workspace, size_t workspace_bytes, void* stream);
+/* Of `count` states (complex64 [count, n, n], device): the hermiticity defect ||rho - rho^+||_F /
+ * ||rho||_F (float64 [count], device; a zero state gives 0) and the trace (complex128 [count],
+ * device), FP64 sums. */
+DQB_API int dqb_state_checks(const void* states, int32_t n, int64_t count, double* hermiticity,
+                             void* trace, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- library info ------------------------------------------------------------- */
 /* Largest n handled by the shared-memory persistent kernel for a jump count. */
