@@ -52,6 +52,22 @@ def _flops_per_rhs(n: int, K: int) -> float:
     return (1 + 2 * K) * 8.0 * n ** 3
 
 
+def _banded_nonzeros(w, precision):
+    """Nonzeros of Hnh and of the jump operators when the dense-storage workload's operators
+    are banded (at most 8 diagonals each: the kernels then work on the nonzeros alone), else
+    None.  The f16x3 kernel multiplies full matrices."""
+    if hasattr(w['H'], 'diags') or precision == 'f16x3':
+        return None
+    H = np.asarray(w['H'])
+    H = H.reshape(-1, *H.shape[-2:])[0]
+    Ls = [np.asarray(L) for L in w['jump_ops']]
+    masks = [(H != 0) | (sum(L.conj().T @ L for L in Ls) != 0)] + [L != 0 for L in Ls]
+    diags = [len(np.unique(np.subtract(*np.nonzero(m)))) for m in masks]
+    if diags[0] > 8 or sum(diags[1:]) > 8 or len(Ls) > 8:
+        return None
+    return int(masks[0].sum()), [int(m.sum()) for m in masks[1:]]
+
+
 def _clock_sampler(path):
     q = ('index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,'
          'clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,'
@@ -338,10 +354,10 @@ def _workload(name, args, rank):
     return w
 
 
-def _kernels_per_launch(path: str, K: int, iterations: int, stepper: str = 'auto') -> int:
+def _kernels_per_launch(path: str, K: int, iterations: int, stepper: str = 'auto', banded=None) -> int:
     """Kernels of this library executed by one solve call."""
     if path == 'dqb_mesolve_dense':
-        return 1  # the persistent kernel (plus a 256-byte memset of its work counter)
+        return 3  # work counters, banded instances, the others
     if path == 'dqb_mesolve_dia':
         if stepper != 'krylov':
             body = 6 * 2 + 4      # 6 x (combine + stencil) + error, control, save, commit
@@ -351,17 +367,20 @@ def _kernels_per_launch(path: str, K: int, iterations: int, stepper: str = 'auto
             init = 9              # set-up, Hnh, rho0, 2 RHS, 2 norms, 2 controls
         return init + body * iterations + 3
     rhs = (2 if K else 1) + 1 + ((K + 1) // 4 if K > 3 else 0)  # L X, sums, symmetrize
+    loop = 1 if banded else rhs  # the stencil alone, or the products
+    # set-up, rho0, diagonals (5 launches), Hnh, 2 x (stencil + products), loop choice
+    init = 2 + 5 + max(1, (K + 3) // 4) + 2 * (1 + rhs) + 1
     if stepper != 'krylov':
-        body = 6 * (1 + rhs) + 4  # 6 x (combine + RHS) + error, control, save, commit
-        init = 3 + 2 * rhs + 5 + (K + 3) // 4
+        body = 6 * (1 + loop) + 4  # 6 x (combine + RHS) + error, control, save, commit
+        init += 5
     else:
-        body = 6 * rhs + 4        # 6 basis RHS + combination, control, save, commit
-        init = 3 + 2 * rhs + 4 + (K + 3) // 4
+        body = 6 * loop + 4        # 6 basis RHS + combination, control, save, commit
+        init += 4
     return init + body * iterations + 3
 
 
 def _roofline(config, precision, n, K, nsteps, mean_ms, B, peaks, which, nsave=0, nacc=None,
-              stepper='auto'):
+              stepper='auto', banded=None):
     """Roofline record of the dominant kernel of a solve launch: `nsteps` (tensor) is the
     attempted RK steps of every instance, `nacc` the accepted ones, `mean_ms` the launch's
     mean duration."""
@@ -405,12 +424,19 @@ def _roofline(config, precision, n, K, nsteps, mean_ms, B, peaks, which, nsave=0
         return roof
     rhs_evals = float((6 * nsteps + 2).sum())
     flops = rhs_evals * _flops_per_rhs(n, K)
+    if banded:  # the products on the nonzeros, and 28 multiply-adds of a state per step
+        flops = rhs_evals * (8.0 * n * (banded[0] + 2 * sum(banded[1])) + 28 * 4.0 * n * n / 6)
     achieved = flops / (mean_ms / 1e3) / 1e12
     peak = peaks.get('bf16_tflops_sustained', peaks.get('bf16_tflops'))
     roof = {'bound': 'tensor', 'achieved': achieved, 'peak': peak, 'unit': 'TFLOP/s',
             'frac': achieved / peak, 'peak_source': f'bf16_tflops_sustained ({which})',
             'traffic': _traffic(config, precision, B, nsteps), 'algorithmic_flops_per_launch': flops}
-    if precision == 'fp32' or (precision in ('tf32x3', 'bf16x3', 'tf32') and n <= 64):
+    if banded:
+        roof['note'] = ('banded operators: the right-hand side is a stencil of their nonzero diagonals '
+                        'on the FP32 CUDA cores, and flops count those; no tensor-core products '
+                        'run.  Bound by latency (n <= 64: two warps per scheduler hold the '
+                        'Runge-Kutta state in registers) or by HBM and L2 (n > 64)')
+    elif precision == 'fp32' or (precision in ('tf32x3', 'bf16x3', 'tf32') and n <= 64):
         roof['note'] = ('products run on the FP32 CUDA-core pipe (SIMT), not the tensor '
                         'pipe; see roofline_fp32_simt')
         if n <= 64 and K > 0:
@@ -536,8 +562,9 @@ def run_b200(args):
     value = world * B * args.steps / (kern / 1e3)
     mean_ms = kern / args.steps
     peaks, which = _peaks()
+    banded = _banded_nonzeros(w, args.precision)
     roof = _roofline(args.config, args.precision, n, K, nsteps, mean_ms, B, peaks, which,
-                     len(w['tsave']), nacc, args.stepper)
+                     len(w['tsave']), nacc, args.stepper, banded)
 
     # ---- e2e: public API from host inputs --------------------------------------------
     e2e = None
@@ -628,7 +655,7 @@ def run_b200(args):
                    'avg_rk_steps': float(nsteps.mean()), 'max_rk_steps': float(nsteps.max())},
         'e2e': e2e,
         'gpu_launches': args.steps * _kernels_per_launch(prep.name, K, int(nsteps.max()),
-                                                         args.stepper),
+                                                         args.stepper, banded),
         'roofline': roof,
         **extra,
         'clocks': clocks,
@@ -690,7 +717,8 @@ def _extra_configs(args, dev, stream, flush, peaks, which):
                     'max_rk_steps': float(nsteps.max()),
                     'stepper': stepper,
                     'roofline': _roofline(cfg, prec, n, len(w['jump_ops']), nsteps, mean_ms, B,
-                                          peaks, which, len(w['tsave']), nacc, stepper)}
+                                          peaks, which, len(w['tsave']), nacc, stepper,
+                                          _banded_nonzeros(w, prec))}
         del prep
         torch.cuda.empty_cache()
     return out
