@@ -557,15 +557,27 @@ __device__ __forceinline__ void band_stencil(const LargeOps& d, int b, const flo
 #pragma unroll
   for (int r = 0; r < NR; ++r) row[r] = min(ti * 32 + t.row(r * NC), n - 1);
   const int col = min(tj * 32 + t.col(0), n - NC);
-  // X[i][s .. s + NC - 1]; beyond the matrix any entry will do, its coefficient is zero
+  // X[i][s .. s + NC - 1]; beyond the matrix any entry will do, its coefficient is zero.
+  // read_all: rows row[r] + di, columns col + dj on.  VEC (n even): col is even, so the
+  // pair is one 16-byte read if dj is even (a pair never straddles the matrix's edge).  The
+  // form is chosen once for all rows, so that no branch keeps a row's reads waiting for
+  // another's.
   auto read = [&](int i, int s, float2 (&x)[NC]) {
     const float2* p = X + min(max(i, 0), n - 1) * n;
-    if (VEC && (s & 1) == 0 && s >= 0 && s < n) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(p + s));
-      x[0] = make_float2(v.x, v.y), x[NC - 1] = make_float2(v.z, v.w);
+#pragma unroll
+    for (int q = 0; q < NC; ++q) x[q] = __ldg(p + min(max(s + q, 0), n - 1));
+  };
+  auto read_all = [&](int di, int dj, float2 (&x)[NR][NC]) {
+    if (VEC && (dj & 1) == 0) {
+      const float2* p = X + min(max(col + dj, 0), n - 2);
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(p + min(max(row[r] + di, 0), n - 1) * n));
+        x[r][0] = make_float2(v.x, v.y), x[r][NC - 1] = make_float2(v.z, v.w);
+      }
     } else {
 #pragma unroll
-      for (int q = 0; q < NC; ++q) x[q] = __ldg(p + min(max(s + q, 0), n - 1));
+      for (int r = 0; r < NR; ++r) read(row[r] + di, col + dj, x[r]);
     }
   };
   float2 A[NR][NC], Bc[NR][NC];
@@ -575,26 +587,20 @@ __device__ __forceinline__ void band_stencil(const LargeOps& d, int b, const flo
     for (int q = 0; q < NC; ++q) A[r][q] = Bc[r][q] = make_float2(0.f, 0.f);
   for (int m = 0; m < R.nh; ++m) {
     const int off = R.hoff[m];
-    float2 hc[NC];
+    float2 hc[NC], hr[NR], x[NR][NC], y[NR][NC];
 #pragma unroll
     for (int q = 0; q < NC; ++q) hc[q] = cconj(__ldg(hd + m * n + col + q));
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      const float2 hr = __ldg(hd + m * n + row[r]);
-      float2 x[NC], y[NC];
-      read(row[r] + off, col, x);
-      if (off != 0) {
-        read(row[r], col + off, y);
-      } else {
+    for (int r = 0; r < NR; ++r) hr[r] = __ldg(hd + m * n + row[r]);
+    read_all(off, 0, x);
+    read_all(0, off, y);
 #pragma unroll
-        for (int q = 0; q < NC; ++q) y[q] = x[q];
-      }
+    for (int r = 0; r < NR; ++r)
 #pragma unroll
       for (int q = 0; q < NC; ++q) {
-        A[r][q] = cfma(hr, x[q], A[r][q]);
-        Bc[r][q] = herm ? cfma(hc[q], y[q], Bc[r][q]) : cfma(y[q], hc[q], Bc[r][q]);
+        A[r][q] = cfma(hr[r], x[r][q], A[r][q]);
+        Bc[r][q] = herm ? cfma(hc[q], y[r][q], Bc[r][q]) : cfma(y[r][q], hc[q], Bc[r][q]);
       }
-    }
   }
   if (!herm) {
 #pragma unroll
@@ -619,21 +625,20 @@ __device__ __forceinline__ void band_stencil(const LargeOps& d, int b, const flo
       if (p1 == p0 + 1) {  // one diagonal: the same X for both sums
         const int off = R.loff[p0];
         const float2 z = make_float2(0.f, 0.f);
-        float2 lc[NC];
+        float2 lc[NC], lr[NR], x[NR][NC];
 #pragma unroll
         for (int q = 0; q < NC; ++q) lc[q] = cconj(__ldg(ld + p0 * n + col + q));
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          const float2 lr = __ldg(ld + p0 * n + row[r]);
-          float2 x[NC];
-          read(row[r] + off, col + off, x);
+        for (int r = 0; r < NR; ++r) lr[r] = __ldg(ld + p0 * n + row[r]);
+        read_all(off, off, x);
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
 #pragma unroll
           for (int q = 0; q < NC; ++q) {
-            const float2 u = cfma(lr, x[q], z), w = cfma(lc[q], x[q], z);
+            const float2 u = cfma(lr[r], x[r][q], z), w = cfma(lc[q], x[r][q], z);
             ga[r][q] = cadd(ga[r][q], cfma(make_float2(half * u.x, half * u.y), lc[q], z));
-            if (herm) gb[r][q] = cadd(gb[r][q], cfma(make_float2(half * w.x, half * w.y), lr, z));
+            if (herm) gb[r][q] = cadd(gb[r][q], cfma(make_float2(half * w.x, half * w.y), lr[r], z));
           }
-        }
         continue;
       }
 #pragma unroll
@@ -708,8 +713,12 @@ __device__ __forceinline__ void band_stencil(const LargeOps& d, int b, const flo
 // k = f(X) of the banded instances.  grid (T (T + 1) / 2, B) in the hermitian form, (T * T, B)
 // in the standard one.  kry = q > 0: a Krylov basis right-hand side, times tau (and sig1 for
 // q = 1).  `mirror`: the hermitian form writes the lower triangle too.
+// Four CTAs per SM (64 registers, a few spills in the branch of several diagonals per jump):
+// the reads' latency is what bounds it.  Transmon x cavity, n = 256, 64 instances, us per
+// launch: 2 CTAs 32, 3 (80 registers) 27, 4 24, 5 48 (spills); a branch around each read
+// in place of read_all, 3 CTAs: 32.
 template <bool VEC>
-__global__ void __launch_bounds__(256) band_rhs_kernel(big::Common c, LargeOps d, int in_sel, int out_k,
+__global__ void __launch_bounds__(256, 4) band_rhs_kernel(big::Common c, LargeOps d, int in_sel, int out_k,
                                                        int need_run, int herm, int kry, int mirror) {
   __shared__ float2 sh[32][33];
   __shared__ BandRec R;

@@ -16,9 +16,9 @@
 // banded instances are computed in FP32, which is at least as exact.)
 //
 // Measured (one B200): transmon x cavity, n = 256, two jumps, 64 instances: 19.0 ms per
-// solve of 12 steps with 3xTF32 products, 5.8 ms with the stencil (30 us a right-hand side
+// solve of 12 steps with 3xTF32 products, 4.5 ms with the stencil (24 us a right-hand side
 // against 196 us).  Bound: instructions and latency of the displaced reads (every operand
-// comes from L1 or L2; 53% of the cycles have no eligible warp); the floor is X read once and k
+// comes from L1 or L2); the floor is X read once and k
 // written once, on the 32 x 32 tiles on and above the diagonal where only the
 // hermitian-half kernels read it.
 #pragma once
