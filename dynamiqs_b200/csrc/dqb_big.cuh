@@ -515,7 +515,7 @@ static __global__ void error_h_kernel(Common c) {
     if (htile_in<VEC>(n, ti, tj, q)) {
       const float ya = cabsf(yv[q]), y1a = cabsf(y1v[q]);
       const double sc = c.o.atol + c.o.rtol * (double)(ya > y1a ? ya : y1a);
-      s += (ex[q] * ex[q] + ey[q] * ey[q]) / (sc * sc);
+      s += ratio(ex[q] * ex[q] + ey[q] * ey[q], sc * sc);
     }
   }
   if (ti != tj) s *= 2.0;
@@ -525,8 +525,19 @@ static __global__ void error_h_kernel(Common c) {
 // Starting-step norms.  phase 0: acc[0] += |y/sc|^2, acc[1] += |k1/sc|^2;
 // phase 1: acc[2] += |(k2 - k1)/sc|^2 (k2 = f(y + h0 k1));
 // phase 2 (Krylov form, k2 holding L k1): acc[2] += |h0 L k1 / sc|^2, the same quantity
-// for a linear right-hand side.
-static __global__ void init_norm_kernel(Common c, int phase) {
+// for a linear right-hand side.  A thread takes four elements at a time, all loads first, and
+// the FP64 divisions are Newton steps (ratio).  One element at a time, latency and the
+// divisions bounded it: n = 4096, 2 instances, 340 -> 164 us a pass; n = 256, 64 instances,
+// 84 -> 30 us (65 with a block per 256 elements, whose atomics then bound it).
+constexpr int kNormElems = 4;
+
+inline dim3 init_norm_grid(const Common& c) {
+  const long long per = (long long)kNormElems * kElemThreads;
+  return dim3((unsigned)std::min<long long>((c.nn + per - 1) / per, 1184), c.B);
+}
+
+template <int phase>
+static __global__ void init_norm_kernel(Common c) {
   __shared__ double red[40];
   const int b = blockIdx.y;
   Inst& I = c.inst[b];
@@ -534,23 +545,30 @@ static __global__ void init_norm_kernel(Common c, int phase) {
   const float2* y = slot(c, b, I.sy);
   const float2* k1 = slot(c, b, I.sk[0]);
   const float2* k2 = slot(c, b, I.sk[1]);
+  const double h0 = I.h0;
   double s0 = 0.0, s1 = 0.0;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < c.nn;
-       e += (long long)gridDim.x * blockDim.x) {
-    const float2 yv = y[e];
-    const double sc = c.o.atol + c.o.rtol * (double)cabsf(yv);
-    const float2 f0 = k1[e];
-    if (phase == 0) {
-      s0 += (double)cabs2f(yv) / (sc * sc);
-      s1 += (double)cabs2f(f0) / (sc * sc);
-    } else if (phase == 1) {
-      const float2 f1 = k2[e];
-      const double dx = (double)f1.x - f0.x, dy = (double)f1.y - f0.y;
-      s0 += (dx * dx + dy * dy) / (sc * sc);
-    } else {
-      const float2 f1 = k2[e];
-      const double dx = I.h0 * f1.x, dy = I.h0 * f1.y;
-      s0 += (dx * dx + dy * dy) / (sc * sc);
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long e0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; e0 < c.nn; e0 += kNormElems * step) {
+    float2 yv[kNormElems], f0[kNormElems], f1[kNormElems];
+#pragma unroll
+    for (int q = 0; q < kNormElems; ++q) {
+      const long long e = min(e0 + q * step, c.nn - 1);  // (beyond the end: read, not counted)
+      yv[q] = y[e];
+      if (phase != 2) f0[q] = k1[e];
+      if (phase != 0) f1[q] = k2[e];
+    }
+#pragma unroll
+    for (int q = 0; q < kNormElems; ++q) {
+      if (e0 + q * step >= c.nn) break;
+      const double sc = c.o.atol + c.o.rtol * (double)cabsf(yv[q]);
+      if (phase == 0) {
+        s0 += ratio((double)cabs2f(yv[q]), sc * sc);
+        s1 += ratio((double)cabs2f(f0[q]), sc * sc);
+      } else {
+        const double dx = phase == 1 ? (double)f1[q].x - f0[q].x : h0 * f1[q].x;
+        const double dy = phase == 1 ? (double)f1[q].y - f0[q].y : h0 * f1[q].y;
+        s0 += ratio(dx * dx + dy * dy, sc * sc);
+      }
     }
   }
   if (phase == 0) {

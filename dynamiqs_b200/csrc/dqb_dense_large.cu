@@ -1381,7 +1381,9 @@ static void init_carveouts() {
     prefer_max_shared(big::load_rho0_kernel);
     prefer_max_shared(big::combine_kernel);
     prefer_max_shared(big::error_kernel);
-    prefer_max_shared(big::init_norm_kernel);
+    prefer_max_shared(big::init_norm_kernel<0>);
+    prefer_max_shared(big::init_norm_kernel<1>);
+    prefer_max_shared(big::init_norm_kernel<2>);
     prefer_max_shared(big::init_ctrl_kernel);
     prefer_max_shared(big::control_kernel);
     prefer_max_shared(big::save_kernel);
@@ -1479,17 +1481,17 @@ static int run_large(const big::Common& c, const LargeOps& d_in, cudaStream_t s,
   }
   at_time(s, 8);
   launch_rhs(s, c, d, B, 0, 0, 0, form, nullptr, nullptr);
-  big::init_norm_kernel<<<ge, T, 0, s>>>(c, 0);
+  big::init_norm_kernel<0><<<big::init_norm_grid(c), T, 0, s>>>(c);
   big::init_ctrl_kernel<<<gi, 128, 0, s>>>(c, 0);
   if (krylov) {
     // the probe f(y + h0 k1) - f(y) of the starting step is h0 L k1 for a linear f
     launch_rhs(s, c, d, B, 3, 1, 0, form, nullptr, nullptr);
-    big::init_norm_kernel<<<ge, T, 0, s>>>(c, 2);
+    big::init_norm_kernel<2><<<big::init_norm_grid(c), T, 0, s>>>(c);
   } else {
     big::launch_combine(s, c, ge, 6);
     at_time(s, 9);
     launch_rhs(s, c, d, B, 2, 1, 0, form, nullptr, nullptr);
-    big::init_norm_kernel<<<ge, T, 0, s>>>(c, 1);
+    big::init_norm_kernel<1><<<big::init_norm_grid(c), T, 0, s>>>(c);
   }
   big::init_ctrl_kernel<<<gi, 128, 0, s>>>(c, 1);
   if (cudaGetLastError() != cudaSuccess) return DQB_ERR_CUDA;

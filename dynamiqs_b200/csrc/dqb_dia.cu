@@ -1394,7 +1394,9 @@ static void init_carveouts() {
     prefer_max_shared(big::load_rho0_kernel);
     prefer_max_shared(big::combine_kernel);
     prefer_max_shared(big::error_kernel);
-    prefer_max_shared(big::init_norm_kernel);
+    prefer_max_shared(big::init_norm_kernel<0>);
+    prefer_max_shared(big::init_norm_kernel<1>);
+    prefer_max_shared(big::init_norm_kernel<2>);
     prefer_max_shared(big::init_ctrl_kernel);
     prefer_max_shared(big::control_kernel);
     prefer_max_shared(big::save_kernel);
@@ -1591,17 +1593,17 @@ static int solve_dia(const dqb_dia_problem* p, const dqb_td_hamiltonian* tdh, co
   big::load_rho0_kernel<<<ge, T, 0, s>>>(c);
   at_time(s, 8);
   launch_rhs_dia(s, c, d, B, rows, 0, 0, 0, nullptr, nullptr, 0, herm);
-  big::init_norm_kernel<<<ge, T, 0, s>>>(c, 0);
+  big::init_norm_kernel<0><<<big::init_norm_grid(c), T, 0, s>>>(c);
   big::init_ctrl_kernel<<<gi, 128, 0, s>>>(c, 0);
   if (krylov) {
     // the probe f(y + h0 k1) - f(y) of the starting step is h0 L k1 for a linear f
     launch_rhs_dia(s, c, d, B, rows, 3, 1, 0, nullptr, nullptr, 0, herm);
-    big::init_norm_kernel<<<ge, T, 0, s>>>(c, 2);
+    big::init_norm_kernel<2><<<big::init_norm_grid(c), T, 0, s>>>(c);
   } else {
     big::launch_combine(s, c, ge, 6);
     at_time(s, 9);
     launch_rhs_dia(s, c, d, B, rows, 2, 1, 0, nullptr, nullptr, 0, herm);
-    big::init_norm_kernel<<<ge, T, 0, s>>>(c, 1);
+    big::init_norm_kernel<1><<<big::init_norm_grid(c), T, 0, s>>>(c);
   }
   big::init_ctrl_kernel<<<gi, 128, 0, s>>>(c, 1);
   if (cudaGetLastError() != cudaSuccess) return DQB_ERR_CUDA;

@@ -350,12 +350,12 @@ int run(const SeOps& d0, int nE, int ntsave, long long B, const void* psi0, cons
   se_load_kernel<<<ge, T, 0, s>>>(c);
   at_time(s, 8);
   launch_rhs(s, c, d, 0, 0, 0);
-  big::init_norm_kernel<<<ge, T, 0, s>>>(c, 0);
+  big::init_norm_kernel<0><<<big::init_norm_grid(c), T, 0, s>>>(c);
   big::init_ctrl_kernel<<<gi, 128, 0, s>>>(c, 0);
   big::combine_kernel<<<ge, T, 0, s>>>(c, 6);
   at_time(s, 9);
   launch_rhs(s, c, d, 2, 1, 0);
-  big::init_norm_kernel<<<ge, T, 0, s>>>(c, 1);
+  big::init_norm_kernel<1><<<big::init_norm_grid(c), T, 0, s>>>(c);
   big::init_ctrl_kernel<<<gi, 128, 0, s>>>(c, 1);
   if (cudaGetLastError() != cudaSuccess) return DQB_ERR_CUDA;
 
