@@ -29,7 +29,8 @@ class Options:
     # control no longer sees a density matrix's far tail and takes fewer, larger steps
     # than the reference (states stay as accurate against an FP64 solution).  'auto' lets
     # the autotuner pick the faster of 'fp32' and 'tf32x3' on the GEMM path and means
-    # 'fp32' elsewhere.  The sparse-DIA kernels always run FP32.
+    # 'fp32' elsewhere.  The sparse-DIA kernels always run FP32, and so do dense operators
+    # of few nonzero diagonals with n > 64 (a stencil in place of the products).
     precision: str = 'fp32'
     # How the sparse-DIA and dense GEMM (n > 64) paths form an RK step (an addition of
     # this library): 'stages' (stage by stage, as diffrax does), 'krylov' (every stage, y1,

@@ -168,7 +168,9 @@ DQB_API size_t dqb_mesolve_dense_workspace_size(int32_t n, int32_t n_jumps, int6
  * MESolveDiffraxIntegrator with Tsit5 / Dopri5 (diffrax_integrator.py:135-147,
  * 283-378).  n <= 64: one persistent CTA per in-flight instance, the whole RK loop on
  * the device (operators and the stage input in shared memory, stages in an
- * L2-resident per-CTA scratch slot).  n > 64 returns DQB_ERR_UNSUPPORTED: use
+ * L2-resident per-CTA scratch slot; hermitian form with at most 8 nonzero diagonals in Hnh
+ * and 8 in the jump operators, found on the device: stages in registers, the products as
+ * stencils).  n > 64 returns DQB_ERR_UNSUPPORTED: use
  * dqb_mesolve_dense_large. */
 DQB_API int dqb_mesolve_dense(const dqb_dense_problem* problem, const dqb_ode_options* options,
                       const dqb_outputs* outputs, void* workspace,
@@ -326,8 +328,9 @@ DQB_API size_t dqb_sesolve_dense_workspace_size(void);
  * psi) and dense output as dqb_mesolve_dense.  The problem is a dqb_dense_problem with
  * n_jumps = 0 and rho0 = psi0 as kets [*, n, 1] (rho0_is_ket and L are ignored); states
  * are kets: complex64 [batch, nsave, n, 1]; expects[b, m, s] = <psi|E_m|psi>
- * (utils/general.py:467-474).  One warp per in-flight instance, H in shared memory, psi
- * and the stages in registers.  n > 128 returns DQB_ERR_UNSUPPORTED. */
+ * (utils/general.py:467-474).  H of at most 8 nonzero diagonals: one warp per
+ * in-flight instance; any other: one CTA per instance, H in shared memory.  psi's stages
+ * are in registers.  n > 128 returns DQB_ERR_UNSUPPORTED. */
 DQB_API int dqb_sesolve_dense(const dqb_dense_problem* problem, const dqb_ode_options* options,
                               const dqb_outputs* outputs, void* workspace, size_t workspace_bytes,
                               void* stream);
