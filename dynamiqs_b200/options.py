@@ -36,8 +36,8 @@ class Options:
     # this library): 'stages' (stage by stage, as diffrax does), 'krylov' (every stage, y1,
     # the error estimate and the dense output as polynomials in hL applied to y, from the
     # basis (hL)^q y, q <= 7: the same method in exact arithmetic, 22 instead of 54 passes
-    # over the state per step, and a rejected step reuses its basis; 1.8x faster on the
-    # coupled-Kerr DIA workload, 1.2x on transmon x cavity, but in FP32 the expanded
+    # over the state per step, and a rejected step reuses its basis; 1.5x faster on the
+    # coupled-Kerr DIA workload, 1.4x on transmon x cavity, but in FP32 the expanded
     # polynomial rounds up to ~5x worse than the stages on stiff problems, still inside
     # the solve's tolerance), or 'auto' (= 'stages').  The n <= 64 kernel, sesolve and
     # the vectorized form run 'stages'.
