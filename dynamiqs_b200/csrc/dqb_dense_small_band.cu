@@ -79,6 +79,7 @@ __device__ __forceinline__ float2 half_cmul(float2 a, float2 x) {
 struct Lists {
   unsigned mask[1 + kMaxK + kMaxM][4];  // nonzero diagonals: H, the jumps, the terms of H(t)
   int ok, flag;
+  int given;       // rho0's triangles differ in rounding: save points at t0 take rho0 itself
   int nh, nk, nl;  // diagonals of Hnh (ascending), jump operators, their diagonals (ascending)
   unsigned long long hpack, lpack;  // their offsets, packed (offset_of)
   int hoff[kMaxH];
@@ -180,6 +181,33 @@ __device__ __forceinline__ void block_sums(double (&v)[N], Shared<T, R>& sh, int
     v[i] = s;
   }
   par ^= 1;
+}
+
+// The first `saved` save points that lie at t0, and the final state where only that is kept
+// and no step was taken (`at_start`), from rho0 as given: the solve has gone by its upper
+// triangle.  A call at the end of a solve, so that its registers cost the solve none.
+template <int T, int R>
+__device__ __noinline__ void save_given(const InstView& a, Shared<T, R>& sh, int saved, bool at_start) {
+  const int n = a.n;
+  int par = 0;
+  __syncthreads();  // the states have been written, the sums read
+  if (!a.save_states && at_start)
+    for (int e = threadIdx.x; e < n * n; e += T * T) a.states[e] = a.rho0[e];
+  for (int s = 0; s < saved && a.tsave[s] <= a.t0; ++s) {
+    if (a.save_states)
+      for (int e = threadIdx.x; e < n * n; e += T * T) a.states[(long long)s * n * n + e] = a.rho0[e];
+    for (int m = 0; m < a.nE; ++m) {
+      double v[2] = {0.0, 0.0};
+      for (int e = threadIdx.x; e < n * n; e += T * T) {
+        const int i = e / n, j = e - i * n;
+        const float2 r = a.rho0[e], eji = __ldg(a.E + (long long)m * n * n + j * n + i);
+        v[0] += (double)eji.x * r.x - (double)eji.y * r.y;
+        v[1] += (double)eji.x * r.y + (double)eji.y * r.x;
+      }
+      block_sums(v, sh, par);
+      if (threadIdx.x == 0) a.expects[m * a.ntsave + s] = make_float2((float)v[0], (float)v[1]);
+    }
+  }
 }
 
 // One instance.  Returns false (to every thread) when the instance is not banded or its
@@ -310,6 +338,7 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
     __syncthreads();
     if (!(asym <= 4.8e-7f * big)) return false;
   }
+  if (tid == 0) ls.given = !a.is_ket && asym != 0.f;
   for (int e = tid; e < 21; e += NT) {
     int s = 1;
     while (e >= s * (s + 1) / 2) ++s;
@@ -759,6 +788,7 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
     __syncthreads();
     copy_out(X, a.states, n);
   }
+  if (ls.given) save_given(a, sh, sidx, !(t > a.t0));
   // every output before the status (see solve_one)
   __threadfence();
   __syncthreads();

@@ -119,3 +119,32 @@ def test_large_mixed_batch_and_tensor_cores(cuda_device):
         assert (got.states[b] - alone[b].states).abs().amax() <= 1e-7
     tc = dq.mesolve(H, Ls, rho, ts, exp_ops=Es, options=dq.Options(precision='tf32x3'))
     _agree(tc, dq.mesolve(H, Ls, rho, ts, exp_ops=Es))
+
+
+@pytest.mark.parametrize('n, batch', [(1, 1), (5, 1), (8, 400), (30, 400), (30, 1), (48, 3), (64, 3)])
+def test_initial_state_is_the_given_one(cuda_device, n, batch):
+    """A rho0 whose triangles differ in the last bits: what is saved at t0 -- state, trace,
+    hermiticity defect, expectation values -- is rho0's own; the later states are those of its
+    upper triangle to a few roundings of rho0's largest entry."""
+    H, Ls, rho, _ = _problem(n, n, batch, [(1,)])
+    rng = np.random.default_rng(n)
+    dust = (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))) * (3e-8 * np.abs(rho).max())
+    rho = (rho + dust).astype(np.complex64)
+    E = (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))).astype(np.complex64)
+    res = dq.mesolve(H, Ls, rho, [0.0, 0.0, 0.2], exp_ops=[E])
+    given = torch.as_tensor(rho).cuda()
+    r = rho.astype(np.complex128)
+    defect = np.linalg.norm(r - r.conj().T) / np.linalg.norm(r)
+    value = np.trace(E.astype(np.complex128) @ r)
+    for s in (0, 1):
+        assert torch.equal(res.states[:, s], given.expand(batch, n, n))
+        # FP64 sums in another order; expectation values are rounded to FP32 once
+        assert (res.checks['hermiticity'][:, s] - defect).abs().max() <= 1e-12
+        assert (res.expects[:, 0, s].to(torch.complex128) - value).abs().max() <= 2 ** -23 * abs(value) + 1e-12
+    upper = (np.triu(rho, 1) + np.triu(rho, 1).conj().T + np.diag(np.diag(rho).real)).astype(np.complex64)
+    ref = dq.mesolve(H, Ls, upper, [0.0, 0.0, 0.2], exp_ops=[E])
+    assert torch.equal(res.states[:, 2], ref.states[:, 2]) and torch.equal(res.infos.nsteps, ref.infos.nsteps)
+    # no step at all: every save point and the final state are rho0
+    assert torch.equal(dq.mesolve(H, Ls, rho, [0.5]).states[:, 0], given.expand(batch, n, n))
+    last = dq.mesolve(H, Ls, rho, [0.5], options=dq.Options(save_states=False))
+    assert torch.equal(last.final_state.reshape(batch, n, n), given.expand(batch, n, n))
