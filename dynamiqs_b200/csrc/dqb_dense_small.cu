@@ -554,6 +554,13 @@ static int grid_for(int NP, int K, long long batch) {
   }
 }
 
+// A launch's CTAs, held to the slots of its workspace: the query counts the CTAs of the
+// constant-H variant, and a variant with less static shared memory can have one more on an SM
+// (n <= 16 with 32 shared matrices of jumps, time-dependent: three against two).
+static int slots_grid(int grid, int NP, size_t workspace_bytes) {
+  return (int)std::min<size_t>(grid, (workspace_bytes - 256) / ((size_t)kSlotMats * NP * NP * sizeof(float2)));
+}
+
 }  // namespace dqb
 
 using namespace dqb;
@@ -653,7 +660,7 @@ extern "C" int dqb_mesolve_dense(const dqb_dense_problem* p, const dqb_ode_optio
   const size_t need = dqb_mesolve_dense_workspace_size(p->n, p->n_jumps, p->batch);
   if (need == 0) return DQB_ERR_UNSUPPORTED;
   if (!workspace || workspace_bytes < need) return DQB_ERR_WORKSPACE_TOO_SMALL;
-  const int grid = grid_for(NP, p->n_jumps, p->batch);
+  const int grid = slots_grid(grid_for(NP, p->n_jumps, p->batch), NP, workspace_bytes);
   cudaStream_t s = (cudaStream_t)stream;
   DenseSmallArgs a = make_args(p, o, out);
   a.counter = (unsigned int*)workspace;
@@ -698,7 +705,7 @@ extern "C" int dqb_mesolve_dense_td(const dqb_dense_problem* p, const dqb_td_ham
   const size_t need = dqb_mesolve_dense_workspace_size(p->n, Keff, p->batch);
   if (need == 0) return DQB_ERR_UNSUPPORTED;
   if (!workspace || workspace_bytes < need) return DQB_ERR_WORKSPACE_TOO_SMALL;
-  const int grid = grid_for<1>(NP, Keff, p->batch);
+  const int grid = slots_grid(grid_for<1>(NP, Keff, p->batch), NP, workspace_bytes);
   cudaStream_t s = (cudaStream_t)stream;
   DenseSmallArgs a = make_args(p, o, out);
   a.counter = (unsigned int*)workspace;
@@ -1285,7 +1292,7 @@ extern "C" int dqb_mesolve_dense_taped(const dqb_dense_problem* p, const dqb_ode
   const size_t need = dqb_mesolve_dense_workspace_size(p->n, p->n_jumps, p->batch);
   if (need == 0) return DQB_ERR_UNSUPPORTED;
   if (!workspace || workspace_bytes < need) return DQB_ERR_WORKSPACE_TOO_SMALL;
-  const int grid = grid_for<2>(NP, p->n_jumps, p->batch);
+  const int grid = slots_grid(grid_for<2>(NP, p->n_jumps, p->batch), NP, workspace_bytes);
   cudaStream_t s = (cudaStream_t)stream;
   DenseSmallArgs a = make_args(p, o, out);
   a.counter = (unsigned int*)workspace;

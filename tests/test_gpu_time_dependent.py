@@ -295,3 +295,55 @@ def test_dense_time_dependent_jump_operators(cuda_device, n):
     err = np.linalg.norm(res.states.cpu().numpy() - ref, axis=(-2, -1)) / np.linalg.norm(ref, axis=(-2, -1))
     assert err.max() < 1e-5, err
     assert abs(int(res.infos.nsteps) - nsteps) <= slack, (int(res.infos.nsteps), nsteps)
+
+
+def test_workspace_holds_the_slots_of_every_kernel(cuda_device):
+    """n <= 16 with 31 jump operators, full matrices: the time-dependent kernel needs less static
+    shared memory than the constant one, and another CTA of it would fit on an SM.  The launch
+    keeps to the slots of the queried workspace: nothing is written beyond it."""
+    import ctypes
+
+    import torch
+
+    from dynamiqs_b200 import _lib
+
+    n, K, B = 16, 31, 450
+    rng = np.random.default_rng(0)
+    g = rng.normal(size=(B, n, n)) + 1j * rng.normal(size=(B, n, n))
+    dev = cuda_device
+    t = lambda x, d=torch.complex64: torch.as_tensor(np.ascontiguousarray(x)).to(dev, d)  # noqa: E731
+    H = t(g + np.conj(np.swapaxes(g, -1, -2)))
+    L = t(0.02 * (rng.normal(size=(1, K, n, n)) + 1j * rng.normal(size=(1, K, n, n))))
+    rho = torch.zeros((n, n), dtype=torch.complex64, device=dev)
+    rho[0, 0] = 1
+    ts, zeros = t([0.0, 0.2], torch.float64), torch.zeros(B, dtype=torch.int32, device=dev)
+    lib = _lib.load()
+    need = lib.dqb_mesolve_dense_workspace_size(n, K + 1, B)
+    ws = torch.full((need + (64 << 20),), 0x5A, dtype=torch.uint8, device=dev)
+    prob = _lib.DenseProblem(n=n, n_jumps=K, n_exp=0, n_tsave=2, batch=B, H=H.data_ptr(), L=L.data_ptr(),
+                             rho0=rho.data_ptr(), rho0_is_ket=0, E=None, tsave=ts.data_ptr(), H_index=None,
+                             L_index=zeros.data_ptr(), rho0_index=zeros.data_ptr())
+    opts = _lib.OdeOptions(method=_lib.METHOD_TSIT5, form=_lib.FORM_HERMITIAN, rtol=1e-6, atol=1e-8, safety=0.9,
+                           factormin=0.2, factormax=5.0, max_steps=100_000, t0=0.0, save_states=1,
+                           check_hermitian=1)
+    out = {}
+    for name in ('td', 'plain'):
+        o = dict(states=torch.zeros((B, 2, n, n), dtype=torch.complex64, device=dev),
+                 infos=torch.zeros((B, 3), dtype=torch.int32, device=dev),
+                 status=torch.full((B,), -1, dtype=torch.int32, device=dev))
+        s = _lib.Outputs(states=o['states'].data_ptr(), expects=None, infos=o['infos'].data_ptr(),
+                         status=o['status'].data_ptr())
+        stream = torch.cuda.current_stream().cuda_stream
+        if name == 'td':  # no terms: the constant problem on the time-dependent kernel
+            terms = (_lib.TdTerm * _lib.TD_MAX_TERMS)()
+            td = _lib.TdHamiltonian(n_terms=0, ops=None, terms=ctypes.cast(terms, ctypes.POINTER(_lib.TdTerm)),
+                                    n_jump_ts=0, jump_ts=None)
+            rc = lib.dqb_mesolve_dense_td(prob, td, opts, s, ws.data_ptr(), need, stream)
+        else:
+            rc = lib.dqb_mesolve_dense(prob, opts, s, ws.data_ptr(), ws.numel(), stream)
+        _lib.check(rc, name)
+        assert (o['status'] == 0).all()
+        assert name == 'plain' or (ws[need:] == 0x5A).all()
+        out[name] = o
+    assert torch.equal(out['td']['infos'], out['plain']['infos'])
+    assert (out['td']['states'] - out['plain']['states']).abs().max() <= 1e-6
