@@ -473,8 +473,10 @@ static int pick_np(int n) { return n <= 16 ? 16 : (n <= 32 ? 32 : (n <= 64 ? 64 
 
 // Padded size of a batched solve: 48 as well (beyond it 32 < n <= 48 would multiply 64 x 64
 // tiles, 1.78 times the work, on one CTA per SM instead of two: full matrices, n = 45, two
-// jumps, standard form, 300 instances: 10.2 against 19.9 ms).  The tape, its adjoint and the
-// ragged classes keep pick_np's three sizes.
+// jumps, standard form, 300 instances: 10.2 against 19.9 ms).  Every batched solve of the same
+// instances takes it -- with a workspace, with the static scratch, taped --, so that they take
+// the same steps and give the same bits.  The rows of the tape, the adjoint, the tensor-core
+// kernel and the ragged classes keep pick_np's three sizes.
 static int pick_np_solve(int n) { return n > 32 && n <= 48 ? 48 : pick_np(n); }
 
 static size_t max_optin_smem() {
@@ -547,9 +549,7 @@ static int grid_for(int NP, int K, long long batch) {
   switch (NP) {
     case 16: return small_grid<16, FEAT>(K, batch);
     case 32: return small_grid<32, FEAT>(K, batch);
-    case 48:
-      if constexpr (FEAT != 2) return small_grid<48, FEAT>(K, batch);  // (no taped variant)
-      return 0;
+    case 48: return small_grid<48, FEAT>(K, batch);
     default: return small_grid<64, FEAT>(K, batch);
   }
 }
@@ -576,7 +576,7 @@ extern "C" int32_t dqb_dense_small_max_n(int32_t n_jumps) {
 
 extern "C" size_t dqb_mesolve_dense_workspace_size(int32_t n, int32_t n_jumps, int64_t batch) {
   if (pick_np(n) == 0 || batch <= 0) return 0;
-  size_t slots = 0;  // the taped and tensor-core solves of the same problem use pick_np's size
+  size_t slots = 0;  // the tensor-core solve of the same problem uses pick_np's size
   for (const int NP : {pick_np(n), pick_np_solve(n)}) {
     const int g = grid_for(NP, n_jumps, batch);
     if (g <= 0) return 0;
@@ -1287,7 +1287,7 @@ extern "C" int dqb_mesolve_dense_taped(const dqb_dense_problem* p, const dqb_ode
     return DQB_ERR_INVALID_ARGUMENT;
   if (!tape || !tape->t || !tape->h || !tape->y || tape->capacity < 1) return DQB_ERR_INVALID_ARGUMENT;
   if (p->batch == 0) return DQB_OK;
-  const int NP = pick_np(p->n);
+  const int NP = pick_np_solve(p->n);
   if (NP == 0 || dqb_dense_small_max_n(p->n_jumps) < NP) return DQB_ERR_UNSUPPORTED;
   const size_t need = dqb_mesolve_dense_workspace_size(p->n, p->n_jumps, p->batch);
   if (need == 0) return DQB_ERR_UNSUPPORTED;
@@ -1302,11 +1302,12 @@ extern "C" int dqb_mesolve_dense_taped(const dqb_dense_problem* p, const dqb_ode
   a.tape_y = (float2*)tape->y;
   a.tape_cap = tape->capacity;
   zero_words_kernel<<<1, 64, 0, s>>>((unsigned int*)workspace, 64);
-  if ((rc = solve_banded(a, a.counter, 2, NP, s))) return rc;
+  if ((rc = solve_banded(a, a.counter, 2, pick_np(p->n), s))) return rc;
   const size_t smem = smem_for(NP, p->n_jumps);
   switch (NP) {
     case 16: mesolve_small_kernel<16, 2><<<grid, kSmallThreads, smem, s>>>(a); break;
     case 32: mesolve_small_kernel<32, 2><<<grid, kSmallThreads, smem, s>>>(a); break;
+    case 48: mesolve_small_kernel<48, 2><<<grid, kSmallThreads, smem, s>>>(a); break;
     default: mesolve_small_kernel<64, 2><<<grid, kSmallThreads, smem, s>>>(a); break;
   }
   return cudaGetLastError() == cudaSuccess ? DQB_OK : DQB_ERR_CUDA;
@@ -1386,13 +1387,13 @@ namespace dqb {
 
 // Bytes of one in-flight instance's scratch slot for dimension n (0 if n > 64).
 size_t small_slot_bytes(int n) {
-  const int NP = pick_np(n);
+  const int NP = pick_np_solve(n);
   return NP ? (size_t)kSlotMats * NP * NP * sizeof(float2) : 0;
 }
 
 // Resident CTAs of the persistent kernel for (n, K, batch) on the current device.
 int small_resident_grid(int n, int K, long long batch) {
-  const int NP = pick_np(n);
+  const int NP = pick_np_solve(n);
   return NP ? grid_for(NP, K, batch) : 0;
 }
 
@@ -1411,7 +1412,7 @@ int small_check_args(const dqb_dense_problem* p, const dqb_ode_options* o, const
 // and grid * small_slot_bytes(n) bytes of slots at `slots` (both device addresses).
 int small_launch_with_scratch(const dqb_dense_problem* p, const dqb_ode_options* o, const dqb_outputs* out,
                               unsigned int* counter, void* slots, int grid, cudaStream_t s) {
-  const int NP = pick_np(p->n);
+  const int NP = pick_np_solve(p->n);
   DenseSmallArgs a = make_args(p, o, out);
   a.counter = counter;
   a.slots = (float2*)slots;
@@ -1420,6 +1421,7 @@ int small_launch_with_scratch(const dqb_dense_problem* p, const dqb_ode_options*
   switch (NP) {
     case 16: mesolve_small_kernel<16><<<grid, kSmallThreads, smem, s>>>(a); break;
     case 32: mesolve_small_kernel<32><<<grid, kSmallThreads, smem, s>>>(a); break;
+    case 48: mesolve_small_kernel<48><<<grid, kSmallThreads, smem, s>>>(a); break;
     default: mesolve_small_kernel<64><<<grid, kSmallThreads, smem, s>>>(a); break;
   }
   return cudaGetLastError() == cudaSuccess ? DQB_OK : DQB_ERR_CUDA;

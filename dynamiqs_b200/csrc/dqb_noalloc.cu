@@ -12,7 +12,7 @@
 // cudaMalloc, cudaFree or an allocating library routine.
 //
 // The array holds a 256-byte work counter followed by per-CTA slots of
-// 9 * NP * NP complex64 (NP = n rounded up to 16, 32 or 64): at n = 64 a slot is
+// 9 * NP * NP complex64 (NP = n rounded up to 16, 32, 48 or 64): at n = 64 a slot is
 // 288 KiB, so at most 28 instances are in flight at once, fewer than the 148 the
 // workspace entry point runs on a B200 -- the results are identical, the throughput lower.
 //

@@ -410,8 +410,12 @@ __device__ void solve_one(Engine& eng, const InstView& a, const CtrlOpts& o, flo
           a.tape_t[idx] = ctl.t;
           a.tape_h[idx] = h;
         }
-        float2* dst = a.tape_y + (a.inst * (long long)a.tape_cap + idx) * NN;
-        for (int e = tid; e < NN; e += blockDim.x) dst[e] = yv[e];
+        constexpr int TP = NP == 48 ? 64 : NP;  // row length of the tape's states
+        float2* dst = a.tape_y + (a.inst * (long long)a.tape_cap + idx) * TP * TP;
+        for (int e = tid; e < TP * TP; e += blockDim.x) {
+          const int i = e / TP, j = e % TP;
+          dst[e] = i < NP && j < NP ? yv[i * NP + j] : make_float2(0.f, 0.f);
+        }
       }
       // dense output at every save time in (t, tnext]
       while (ctl.save_idx < a.ntsave && a.tsave[ctl.save_idx] <= ctl.tnext) {

@@ -199,7 +199,7 @@ DQB_API int dqb_lindblad_rhs_dense_prec(const dqb_dense_problem* problem, int32_
  * array of DQB_NOALLOC_SCRATCH_BYTES that every GPU loading the library keeps until the
  * process exits; nothing is allocated or freed.  At most
  * (DQB_NOALLOC_SCRATCH_BYTES - 256) / (9 * NP * NP * 8) instances run at once (NP = n
- * rounded up to 16, 32 or 64: 28 at n = 64), so results equal dqb_mesolve_dense's but
+ * rounded up to 16, 32, 48 or 64: 28 at n = 64), so results equal dqb_mesolve_dense's but
  * throughput is lower.  n > 64 returns DQB_ERR_UNSUPPORTED; a problem whose single-instance
  * scratch exceeds the array returns DQB_ERR_SCRATCH_TOO_SMALL.  The first call on each
  * device looks up the array's address (cudaGetSymbolAddress) and should come before any

@@ -202,3 +202,26 @@ def test_banded_adjoint_same_as_products(cuda_device, n, jumps, ket):
     mixed[1][0] += np.complex64(1e-25)
     for a, b in zip(grads(mixed[0]), grads(mixed[1])):
         assert (a - b).abs().max() <= 64 * 2 ** -24 * b.abs().max()
+
+
+def _full_problem(n, batch, seed=0):
+    rng = np.random.default_rng(seed)
+    g = rng.normal(size=(batch, n, n)) + 1j * rng.normal(size=(batch, n, n))
+    H = ((g + np.conj(np.swapaxes(g, -1, -2))) / 4).astype(np.complex64)
+    L = (0.3 * (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))) / np.sqrt(n)).astype(np.complex64)
+    y = rng.normal(size=(n, 1)) + 1j * rng.normal(size=(n, 1))
+    E = (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))).astype(np.complex64)
+    return H, L, (y / np.linalg.norm(y)).astype(np.complex64), (E + E.conj().T) / 2
+
+
+@pytest.mark.parametrize('n', [16, 33, 40, 48, 49])
+def test_taped_solve_is_the_solve(cuda_device, n):
+    """The taped solve takes the steps of the plain one: equal bits, full matrices, on both
+    sides of the padded sizes."""
+    H, L, psi, E = _full_problem(n, 12)
+    ts = np.linspace(0.0, 0.8, 9)
+    plain = dq.mesolve(H, [L], psi, ts, exp_ops=[E])
+    taped = dq.mesolve(torch.as_tensor(H).requires_grad_(), [L], psi, ts, exp_ops=[E])
+    assert torch.equal(plain.infos.nsteps, taped.infos.nsteps)
+    assert torch.equal(plain.infos.naccepted, taped.infos.naccepted)
+    assert torch.equal(plain.states, taped.states.detach()) and torch.equal(plain.expects, taped.expects.detach())

@@ -110,3 +110,32 @@ def test_noalloc_rejects_sizes_beyond_its_kernel(cuda_device):
     prob.n = 65
     _, s = _outputs(2, nt)
     assert lib.dqb_mesolve_dense_noalloc(prob, opts, s, None) == _lib.DQB_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize('n', [16, 33, 40, 48, 49])
+def test_noalloc_full_matrices_same_bits(cuda_device, n):
+    """Full matrices on both sides of the padded sizes: the bits of the workspace entry point,
+    with more instances than the static array has slots."""
+    import dynamiqs_b200 as dq
+    from dynamiqs_b200.mesolve import MESolveB200Integrator, make_batch_plan
+
+    rng = np.random.default_rng(n)
+    g = rng.normal(size=(60, n, n)) + 1j * rng.normal(size=(60, n, n))
+    H = ((g + np.conj(np.swapaxes(g, -1, -2))) / 4).astype(np.complex64)
+    L = (0.3 * (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))) / np.sqrt(n)).astype(np.complex64)
+    E = (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))).astype(np.complex64)
+    E = (E + E.conj().T) / 2
+    psi = (rng.normal(size=(n, 1)) + 1j * rng.normal(size=(n, 1))).astype(np.complex64)
+    psi /= np.linalg.norm(psi)
+    integ = MESolveB200Integrator(ts=np.linspace(0.0, 0.5, 4), y0=psi, method=dq.Tsit5(), gradient=None,
+                                  options=dq.Options(), H=H, Ls=[L], Es=[E],
+                                  plan=make_batch_plan(H, [L], psi, True))
+    prep = integ.prepare().launch()
+    want = {k: prep.bufs[k].clone() for k in ('states', 'expects', 'infos')}
+    for k in want:
+        prep.bufs[k].zero_()
+    lib = _lib.load()
+    _lib.check(lib.dqb_mesolve_dense_noalloc(prep.prob, integ._ode_options(), prep.outs,
+                                             torch.cuda.current_stream().cuda_stream), 'noalloc')
+    for k in want:
+        assert torch.equal(prep.bufs[k], want[k])
