@@ -34,27 +34,35 @@ def needs_autograd(H, jump_ops, rho0) -> bool:
         _is_grad_tensor(H) or _is_grad_tensor(rho0) or any(_is_grad_tensor(L) for L in jump_ops))
 
 
-def _solve_taped(integ, lib):
-    """Taped solve: a first solve tells how many steps each instance accepts, the second
-    (the same deterministic kernel) records them."""
-    import torch
+def _accepted(prep) -> int:
+    """The most steps that an instance of the last launch accepted (waits for it)."""
+    return int(prep.bufs['infos'].cpu().numpy()[:, 1].max(initial=0))
 
+
+def _solve_taped(integ, lib):
+    """Taped solve: a plain solve tells how many steps to make room for, the taped one
+    records them."""
     prep = integ._prepare_dense(lib, 'small')
     prep.launch()
-    cap = max(int(prep.bufs['infos'][:, 1].max().item()), 1)
+    _record(integ, lib, prep, max(_accepted(prep), 1))
+    return prep
+
+
+def _record(integ, lib, prep, cap) -> None:
+    """Launches the taped solve with room for ``cap`` steps per instance."""
+    import torch
+
     B = integ.plan.batch
-    n = prep.prob.n
     dev = prep.dev
     tape_t = torch.empty((B, cap), dtype=torch.float64, device=dev)
     tape_h = torch.empty((B, cap), dtype=torch.float64, device=dev)
-    tape_y = torch.empty(lib.dqb_mesolve_dense_tape_bytes(n, cap, B), dtype=torch.uint8, device=dev)
+    tape_y = torch.empty(lib.dqb_mesolve_dense_tape_bytes(prep.prob.n, cap, B), dtype=torch.uint8, device=dev)
     tape = _lib.Tape(t=tape_t.data_ptr(), h=tape_h.data_ptr(), y=tape_y.data_ptr(), capacity=cap)
     rc = lib.dqb_mesolve_dense_taped(prep.prob, integ._ode_options(), prep.outs, tape,
                                      prep.bufs['workspace'].data_ptr(), prep.ws_bytes,
                                      torch.cuda.current_stream(dev).cuda_stream)
     _lib.check(rc, 'dqb_mesolve_dense_taped')
     prep.bufs['tape'] = (tape, tape_t, tape_h, tape_y)
-    return prep
 
 
 def _jump_grads(grad_L, plan, Lts, cartesian, n, dev):
@@ -160,5 +168,11 @@ def mesolve_autograd(H, jump_ops, rho0, tsave, *, exp_ops, method, gradient, opt
             return (gH, gr, *gL)
 
     states, expects = _Solve.apply(Ht, rt, *Lts)
+    # The taped solve's own counts decide whether the tape holds every step: it always runs in
+    # FP32, and a plain solve of another precision may take fewer.  (Read here, where the
+    # result waits for the solve anyway.)
+    while (taken := _accepted(prep)) > prep.bufs['tape'][0].capacity:
+        _record(integ, lib, prep, taken)
+        states, expects = _Solve.apply(Ht, rt, *Lts)
     # the rest of the result (shapes, infos, checks) as for any solve
     return integ._result(states, expects, prep.bufs['infos'], prep.bufs['status'])

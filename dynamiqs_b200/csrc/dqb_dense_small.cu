@@ -817,7 +817,8 @@ constexpr int kAdjMats = 23;  // X_1..7, k_1..6 (+1 spare), kappa_1..7, xi, lamb
 
 struct AdjArgs {
   DenseSmallArgs p;              // operators, indices, E, tsave, method, form, t0
-  const int* nacc;               // [batch] accepted steps of each instance (forward infos)
+  const int* nacc;               // [batch] accepted steps of each instance (forward infos); an
+                                 // instance with more than the tape holds gets NaN gradients
   const float2* gstates;         // [batch, nsave, n, n] cotangents of the saved states, or null
   const float2* gexpects;        // [batch, nE, ntsave] cotangents of the expectation values, or null
   float2* grad_rho0;             // [batch, n, n] (or [batch, n] for kets)
@@ -895,8 +896,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) mesolve_adjoint_kernel(AdjAr
     const long long nn = (long long)n * n;
     float2* gH = A.grad_H + b * nn;
     float2* gL = A.grad_L + b * K * nn;
-    for (long long e = tid; e < nn; e += blockDim.x) gH[e] = make_float2(0.f, 0.f);
-    for (long long e = tid; e < K * nn; e += blockDim.x) gL[e] = make_float2(0.f, 0.f);
+    const bool lost = A.nacc[b] > a.tape_cap;  // (see AdjArgs::nacc)
+    const float2 none = lost ? make_float2(NAN, NAN) : make_float2(0.f, 0.f);
+    for (long long e = tid; e < nn; e += blockDim.x) gH[e] = none;
+    for (long long e = tid; e < K * nn; e += blockDim.x) gL[e] = none;
     load_padded<NP>(sH, v.H, n);
     for (int k = 0; k < K; ++k) load_padded<NP>(sL + k * MAT, v.L + (long long)k * nn, n);
     __syncthreads();
@@ -906,12 +909,12 @@ __global__ void __launch_bounds__(kSmallThreads, 1) mesolve_adjoint_kernel(AdjAr
     // lambda: the final state's cotangent when only it is saved, else zero
     for (int e = tid; e < NN; e += blockDim.x) {
       const int i = e / NP, j = e % NP;
-      float2 g = make_float2(0.f, 0.f);
-      if (!a.o.save_states && A.gstates && i < n && j < n) g = A.gstates[b * nn + i * n + j];
+      float2 g = none;
+      if (!lost && !a.o.save_states && A.gstates && i < n && j < n) g = A.gstates[b * nn + i * n + j];
       lam[e] = g;
     }
     int sp = a.ntsave - 1;  // saves are taken from the last one backwards
-    const int N = min(A.nacc[b], a.tape_cap);
+    const int N = lost ? 0 : A.nacc[b];
     for (int st = N - 1; st >= 0; --st) {
       const double t = v.tape_t[st], h = v.tape_h[st];
       const float2* y = a.tape_y + (b * (long long)a.tape_cap + st) * NN;
@@ -1102,13 +1105,15 @@ __global__ void __launch_bounds__(kSmallThreads, NP <= 16 ? 2 : 1) mesolve_adjoi
     if (tid == 0) marks[b] = bl.ok ? 0 : band::kPending;
     if (!bl.ok) continue;  // (every thread reads bl.ok before the next instance's barriers)
     const int nsave = a.o.save_states ? a.ntsave : 1;
+    const bool lost = A.nacc[b] > a.tape_cap;  // (see AdjArgs::nacc)
+    const float2 none = lost ? make_float2(NAN, NAN) : make_float2(0.f, 0.f);
     float2 lam[R][R], gH[R][R], gL[KR][R][R];
-    zero_tile<NP>(gH);
-#pragma unroll
-    for (int k = 0; k < KR; ++k) zero_tile<NP>(gL[k]);
     each([&](int r, int c, int i, int j) {
-      lam[r][c] = make_float2(0.f, 0.f);
-      if (!a.o.save_states && A.gstates && i < n && j < n) lam[r][c] = A.gstates[b * nn + i * n + j];
+      gH[r][c] = none;
+#pragma unroll
+      for (int k = 0; k < KR; ++k) gL[k][r][c] = none;
+      lam[r][c] = none;
+      if (!lost && !a.o.save_states && A.gstates && i < n && j < n) lam[r][c] = A.gstates[b * nn + i * n + j];
     });
     // cotangent of save point sp on element (i, j)
     auto save_cot = [&](int sp, int i, int j) {
@@ -1121,7 +1126,7 @@ __global__ void __launch_bounds__(kSmallThreads, NP <= 16 ? 2 : 1) mesolve_adjoi
       return g;
     };
     int sp = a.ntsave - 1;  // saves are taken from the last one backwards
-    const int N = min(A.nacc[b], a.tape_cap);
+    const int N = lost ? 0 : A.nacc[b];
     for (int st = N - 1; st >= 0; --st) {
       const double t = v.tape_t[st], h = v.tape_h[st];
       const float2* Y = a.tape_y + (b * (long long)a.tape_cap + st) * tape_np * tape_np;

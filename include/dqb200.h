@@ -253,7 +253,8 @@ DQB_API int dqb_mesolve_dense_taped(const dqb_dense_problem* problem, const dqb_
 DQB_API size_t dqb_mesolve_dense_adjoint_workspace_size(int32_t n, int32_t n_jumps, int64_t batch);
 
 /* The adjoint pass: `naccepted` is the device int32 [batch] of accepted steps the taped
- * solve reported (infos[:, 1]); every one of them must be on the tape. */
+ * solve reported (infos[:, 1]); every one of them must be on the tape (an instance with more
+ * of them than the tape's capacity gets NaN gradients). */
 DQB_API int dqb_mesolve_dense_adjoint(const dqb_dense_problem* problem, const dqb_ode_options* options,
                                       const dqb_tape* tape, const int32_t* naccepted,
                                       const dqb_cotangents* cotangents, const dqb_gradients* gradients,

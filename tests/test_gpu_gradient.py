@@ -225,3 +225,74 @@ def test_taped_solve_is_the_solve(cuda_device, n):
     assert torch.equal(plain.infos.nsteps, taped.infos.nsteps)
     assert torch.equal(plain.infos.naccepted, taped.infos.naccepted)
     assert torch.equal(plain.states, taped.states.detach()) and torch.equal(plain.expects, taped.expects.detach())
+
+
+def _grads(H, L, psi, E, **kw):
+    leaves = [torch.as_tensor(v).clone().requires_grad_() for v in (H, L, psi)]
+    res = dq.mesolve(leaves[0], [leaves[1]], leaves[2], [0.0, 0.2, 0.5], exp_ops=[E], **kw)
+    return torch.autograd.grad(res.expects.real.sum() + res.states[..., 0, 1].real.sum(), leaves)
+
+
+@pytest.mark.parametrize('n, banded', [(12, True), (40, False), (40, True)])
+def test_tape_grows_to_the_steps_taken(cuda_device, monkeypatch, n, banded):
+    """A first guess of the capacity that is too small (one step) gives the gradient of an
+    ample tape, to the bit."""
+    from dynamiqs_b200.mesolve import PreparedSolve
+
+    H, L, psi, E = _full_problem(n, 1)
+    if banded:
+        H, L = np.triu(np.tril(H, 1), -1), np.triu(np.tril(L, 1), 1)
+    want = _grads(H, L, psi, E)
+    launch = PreparedSolve.launch
+
+    def short(self, *a, **k):
+        launch(self, *a, **k)
+        self.bufs['infos'][:, 1] = 1
+        return self
+
+    monkeypatch.setattr(PreparedSolve, 'launch', short)
+    for a, b in zip(_grads(H, L, psi, E), want):
+        assert torch.equal(a, b)
+
+
+def test_gradient_with_a_tensor_core_option(cuda_device):
+    """The taped solve runs in FP32 whatever `precision` asks of the plain one, whose step
+    counts may differ: the gradient is that of FP32."""
+    H, L, psi, E = _full_problem(40, 1)
+    got = _grads(H, L, psi, E, options=dq.Options(precision='f16x3'))
+    for a, b in zip(got, _grads(H, L, psi, E)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize('n, banded', [(12, True), (40, False)])
+def test_adjoint_of_a_short_tape_is_nan(cuda_device, n, banded):
+    """Steps that the tape does not hold make the instance's gradients NaN, not those of
+    the steps that it holds; the other instances keep theirs."""
+    import ctypes
+
+    from dynamiqs_b200 import _lib
+    from dynamiqs_b200.autodiff import _solve_taped
+    from dynamiqs_b200.mesolve import MESolveB200Integrator, make_batch_plan
+
+    H, L, psi, E = _full_problem(n, 2)
+    if banded:
+        H, L = np.triu(np.tril(H, 1), -1), np.triu(np.tril(L, 1), 1)
+    integ = MESolveB200Integrator(ts=np.array([0.0, 0.4]), y0=psi, method=dq.Tsit5(), gradient=None,
+                                  options=dq.Options(), H=H, Ls=[L], Es=[E],
+                                  plan=make_batch_plan(H, [L], psi, True))
+    lib = _lib.load()
+    prep = _solve_taped(integ, lib)
+    nacc = prep.bufs['infos'][:, 1].contiguous()
+    nacc[1] = prep.bufs['tape'][0].capacity + 1
+    c64 = torch.complex64
+    out = [torch.zeros(s, dtype=c64, device='cuda') for s in ((2, n), (2, n, n), (2, 1, n, n))]
+    ge = torch.ones((2, 1, 2), dtype=c64, device='cuda')
+    size = lib.dqb_mesolve_dense_adjoint_workspace_size(n, 1, 2)
+    ws = torch.empty(size, dtype=torch.uint8, device='cuda')
+    grads = _lib.Gradients(rho0=out[0].data_ptr(), H=out[1].data_ptr(), L=out[2].data_ptr())
+    _lib.check(lib.dqb_mesolve_dense_adjoint(
+        prep.prob, integ._ode_options(), prep.bufs['tape'][0], ctypes.c_void_p(nacc.data_ptr()),
+        _lib.Cotangents(states=None, expects=ge.data_ptr()), grads, ws.data_ptr(), size,
+        torch.cuda.current_stream().cuda_stream), 'adjoint')
+    for g in out:
+        assert torch.isfinite(torch.view_as_real(g[0])).all() and torch.isnan(g[1].real).all()
