@@ -11,7 +11,8 @@
 // instance if there are at most kMaxH and kMaxL of them; any other instance (full matrices,
 // a rho0 that is not hermitian to rounding, more jumps than the tables hold) is marked in
 // `pend` and left to the product kernel, which runs next on the stream and takes the marked
-// instances only.  Nothing is decided on the host and no result depends on the batch.
+// instances only.  The host decides on the thread layout alone, by the size of the batch, and
+// no result depends on it (block_sums).
 //
 // What bounds it: with the products gone a step is short, and the 27 reads of y and the
 // stages that the combinations of a step make would dominate from L2 (where the product
@@ -91,7 +92,7 @@ struct Shared {
   using G = Geo<T, R>;
   Lists ls;
   double a21[21];             // a[s][j], j < s, row by row
-  double red[2][4 * G::NW];   // two sets, used in turn
+  double red[2][4 * (T == 16 ? 128 : 2)];  // two sets, used in turn (block_sums)
   float cf[G::NW][24];        // each warp's copy of the stage coefficients h a[s][j]
   double inv_nn, t1;
   long long inst;
@@ -160,27 +161,92 @@ __device__ inline void build_lists(Lists& ls, int n, int K, int M) {
   ls.ok = 1;
 }
 
-// Block sum of N values; every thread gets all of them.  One barrier: `par` selects the set
-// of partial sums, used in turn, so a set is rewritten only after a barrier that every
-// reader of it has passed.
-template <int T, int R, int N>
-__device__ __forceinline__ void block_sums(double (&v)[N], Shared<T, R>& sh, int& par) {
-  constexpr int NW = Geo<T, R>::NW;
+// Block sums over the elements.  Their order is the same in both thread layouts, so that a
+// result does not depend on the layout, which the size of the batch chooses: elements of one
+// place in the 16 x 16 blocks, tile by tile; the place's four images in the 8 x 8 blocks; then
+// the 8 x 8 places, as a tree over rows 0-3 and one over rows 4-7.  With T = 8 a thread is an
+// 8 x 8 place (the parity of its tile's row and column gives the image) and the trees are
+// shuffles before the barrier; with T = 16 it is one image, and they follow the barrier that the
+// exchange of images needs.  (An order that suits T = 16 better, the rows last, cost T = 8 up
+// to 9% of a solve.)
+
+// Before the barrier: N quantities to red, where add(e, r, c) adds the thread's element of tile
+// (r, c) to e, for the tiles r <= c (or, not kUpper, all).
+template <int T, int R, int N, bool kUpper, class Add>
+__device__ __forceinline__ void sums_begin(double* red, Add add) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // the sums over the tiles (r, c) of parity (a, b), or over all
+  auto tiles = [&](double (&e)[N], int a, int b) {
+    constexpr int kStep = T == 16 ? 1 : 2;
 #pragma unroll
-  for (int i = 0; i < N; ++i) v[i] = warp_sum(v[i]);
-  if ((threadIdx.x & 31) == 0) {
+    for (int i = 0; i < N; ++i) e[i] = 0.0;
 #pragma unroll
-    for (int i = 0; i < N; ++i) sh.red[par][i * NW + (threadIdx.x >> 5)] = v[i];
+    for (int r = a; r < R; r += kStep)
+#pragma unroll
+      for (int c = b; c < R; c += kStep)
+        if (!kUpper || r <= c) add(e, r, c);
+  };
+  double e[N];
+  tiles(e, 0, 0);
+  if constexpr (T == 16) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      e[i] += __shfl_xor_sync(0xffffffffu, e[i], 8);  // the images in a block's two halves of a row
+      if ((lane & 8) == 0) red[i * 128 + (threadIdx.x >> 4) * 8 + (lane & 7)] = e[i];
+    }
+  } else {
+    double f[N], g[N];
+    tiles(f, 0, 1);
+#pragma unroll
+    for (int i = 0; i < N; ++i) g[i] = e[i] + f[i];
+    tiles(e, 1, 0);
+    tiles(f, 1, 1);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const double x = warp_sum(g[i] + (e[i] + f[i]));
+      if (lane == 0) red[i * 2 + warp] = x;
+    }
   }
+}
+
+// After it: quantity i (to every thread of the calling warps).
+template <int T>
+__device__ __forceinline__ double sums_end(const double* red, int i) {
+  if (T == 8) return red[i * 2] + red[i * 2 + 1];
+  const double* p = red + i * 128 + (threadIdx.x & 31);
+  return warp_sum(p[0] + p[64]) + warp_sum(p[32] + p[96]);
+}
+
+// Sums to every thread.  One barrier: `par` selects the set of partial sums, used in turn, so a
+// set is rewritten only after a barrier that every reader of it has passed.
+template <int T, int R, int N, class Add>
+__device__ __forceinline__ void block_sums(double (&v)[N], Shared<T, R>& sh, int& par, Add add) {
+  double* red = sh.red[par];
+  par ^= 1;
+  sums_begin<T, R, N, true>(red, add);
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < N; ++i) {
-    double s = 0.0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) s += sh.red[par][i * NW + w];
-    v[i] = s;
-  }
+  for (int i = 0; i < N; ++i) v[i] = sums_end<T>(red, i);
+}
+
+// Expectation values `m` on of save point `sidx`, up to two: add(e, E, r, c) adds the thread's
+// element of tile (r, c) to the value of operator E.  One barrier.
+template <int T, int R, bool kUpper, class Add>
+__device__ __forceinline__ void expect_sums(const InstView& a, Shared<T, R>& sh, int& par, int m, int sidx, Add add) {
+  double* red = sh.red[par];
   par ^= 1;
+  const int ops = min(a.nE - m, 2);
+#pragma unroll 1
+  for (int k = 0; k < ops; ++k) {
+    const float2* E = a.E + (long long)(m + k) * a.n * a.n;
+    sums_begin<T, R, 2, kUpper>(red + k * (T == 16 ? 256 : 4), [&](double (&e)[2], int r, int c) { add(e, E, r, c); });
+  }
+  __syncthreads();
+  const int i = T == 16 ? threadIdx.x >> 5 : threadIdx.x;  // a warp, or a thread, per part
+  if (i >= 2 * ops) return;
+  const double x = sums_end<T>(red, i);
+  if (T == 8 || (threadIdx.x & 31) == 0)
+    reinterpret_cast<float*>(a.expects + (long long)(m + (i >> 1)) * a.ntsave + sidx)[i & 1] = (float)x;
 }
 
 // The first `saved` save points that lie at t0, and the final state where only that is kept
@@ -196,17 +262,14 @@ __device__ __noinline__ void save_given(const InstView& a, Shared<T, R>& sh, int
   for (int s = 0; s < saved && a.tsave[s] <= a.t0; ++s) {
     if (a.save_states)
       for (int e = threadIdx.x; e < n * n; e += T * T) a.states[(long long)s * n * n + e] = a.rho0[e];
-    for (int m = 0; m < a.nE; ++m) {
-      double v[2] = {0.0, 0.0};
-      for (int e = threadIdx.x; e < n * n; e += T * T) {
-        const int i = e / n, j = e - i * n;
-        const float2 r = a.rho0[e], eji = __ldg(a.E + (long long)m * n * n + j * n + i);
-        v[0] += (double)eji.x * r.x - (double)eji.y * r.y;
-        v[1] += (double)eji.x * r.y + (double)eji.y * r.x;
-      }
-      block_sums(v, sh, par);
-      if (threadIdx.x == 0) a.expects[m * a.ntsave + s] = make_float2((float)v[0], (float)v[1]);
-    }
+    for (int m = 0; m < a.nE; m += 2)
+      expect_sums<T, R, false>(a, sh, par, m, s, [&](double (&e)[2], const float2* E, int r, int c) {
+        const int i = threadIdx.x / T + T * r, j = threadIdx.x % T + T * c;
+        if (i >= n || j >= n) return;
+        const float2 u = a.rho0[i * n + j], eji = __ldg(E + j * n + i);
+        e[0] += (double)eji.x * u.x - (double)eji.y * u.y;
+        e[1] += (double)eji.x * u.y + (double)eji.y * u.x;
+      });
   }
 }
 
@@ -329,11 +392,11 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
     // the upper triangle stands for the matrix only when the two agree to rounding
     big = warp_max(big);
     asym = warp_max(asym);
-    if (lane == 0) sh.red[0][warp] = big, sh.red[0][G::NW + warp] = asym;
+    if (lane == 0) sh.red[0][2 * warp] = big, sh.red[0][2 * warp + 1] = asym;
     __syncthreads();
     for (int w = 0; w < G::NW; ++w) {
-      big = fmaxf(big, (float)sh.red[0][w]);
-      asym = fmaxf(asym, (float)sh.red[0][G::NW + w]);
+      big = fmaxf(big, (float)sh.red[0][2 * w]);
+      asym = fmaxf(asym, (float)sh.red[0][2 * w + 1]);
     }
     __syncthreads();
     if (!(asym <= 4.8e-7f * big)) return false;
@@ -350,6 +413,7 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
   }
   __syncthreads();
   double t = a.t0, tnext = t, h = 0.0, dt_prop = 0.0;
+  auto tile_of = [](int r, int c) { return r * R - r * (r - 1) / 2 + c - r; };  // of the upper tiles, row by row
   int made_jump = 0, xb = 0, par = 0, sidx = 0, status = DQB_INST_OK;
   long long nsteps = 0, nacc = 0;
   const int nh = ls.nh, nk = ls.nk;
@@ -396,37 +460,19 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
       copy_out(X, a.states + (long long)sidx * n * n, n);
     }
 #pragma unroll 1
-    for (int m0 = 0; m0 < a.nE; m0 += 2) {
-      double e[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-      for (int mm = 0; mm < 2; ++mm) {
-        if (m0 + mm < a.nE) {
-          const float2* E = a.E + (long long)(m0 + mm) * n * n;
-          int q = 0;
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int c = r; c < R; ++c, ++q) {
-              const int i = ty + T * r, j = tx + T * c;
-              if ((own >> q) & 1u) {
-                const float2 eji = __ldg(E + j * n + i);
-                e[2 * mm] += (double)eji.x * u[q].x - (double)eji.y * u[q].y;
-                e[2 * mm + 1] += (double)eji.x * u[q].y + (double)eji.y * u[q].x;
-                if ((strict >> q) & 1u) {
-                  const float2 eij = __ldg(E + i * n + j);
-                  e[2 * mm] += (double)eij.x * u[q].x + (double)eij.y * u[q].y;
-                  e[2 * mm + 1] += (double)eij.y * u[q].x - (double)eij.x * u[q].y;
-                }
-              }
-            }
+    for (int m = 0; m < a.nE; m += 2)
+      expect_sums<T, R, true>(a, sh, par, m, sidx, [&](double (&e)[2], const float2* E, int r, int c) {
+        const int q = tile_of(r, c), i = ty + T * r, j = tx + T * c;
+        if (!((own >> q) & 1u)) return;
+        const float2 eji = __ldg(E + j * n + i);
+        e[0] += (double)eji.x * u[q].x - (double)eji.y * u[q].y;
+        e[1] += (double)eji.x * u[q].y + (double)eji.y * u[q].x;
+        if ((strict >> q) & 1u) {
+          const float2 eij = __ldg(E + i * n + j);
+          e[0] += (double)eij.x * u[q].x + (double)eij.y * u[q].y;
+          e[1] += (double)eij.y * u[q].x - (double)eij.x * u[q].y;
         }
-      }
-      block_sums(e, sh, par);
-      if (tid == 0) {
-        a.expects[m0 * a.ntsave + sidx] = make_float2((float)e[0], (float)e[1]);
-        if (m0 + 1 < a.nE) a.expects[(m0 + 1) * a.ntsave + sidx] = make_float2((float)e[2], (float)e[3]);
-      }
-    }
+      });
     ++sidx;
   };
 
@@ -459,8 +505,8 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
     // order, with the same roundings, as the product kernel's (which adds the zeros in
     // between): Hnh X by ascending column of Hnh; S onto A and B of a 16 x 16 diagonal
     // block, and twice onto B of the others (the block below the diagonal, whose mirror this
-    // is).  With X hermitian to the last bit the two kernels agree to the last bit, and
-    // with them every accept or reject decision.
+    // is).  With X hermitian to the last bit the two kernels' right-hand sides agree to the last
+    // bit; the FP64 norms, which decide on steps, are added up in another order (block_sums).
     float2 A[Q], B[Q], S[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q) A[q] = B[q] = S[q] = make_float2(0.f, 0.f);
@@ -606,33 +652,29 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
   rhs(t);
   store_k1(v);
   {
-    double sm[2] = {0.0, 0.0};
-#pragma unroll
-    for (int q = 0; q < Q; ++q)
-      if ((own >> q) & 1u) {
-        const double sc = o.atol + o.rtol * (double)cabsf(y[q * NT]), w = (strict >> q) & 1u ? 2.0 : 1.0;
-        sm[0] += w * (double)cabs2f(y[q * NT]) / (sc * sc);
-        sm[1] += w * (double)cabs2f(v[q]) / (sc * sc);
-      }
-    block_sums(sm, sh, par);
+    double sm[2], s2[1];
+    block_sums(sm, sh, par, [&](double (&e)[2], int r, int c) {
+      const int q = tile_of(r, c);
+      if (!((own >> q) & 1u)) return;
+      const double sc = o.atol + o.rtol * (double)cabsf(y[q * NT]), w = (strict >> q) & 1u ? 2.0 : 1.0;
+      e[0] += w * (double)cabs2f(y[q * NT]) / (sc * sc);
+      e[1] += w * (double)cabs2f(v[q]) / (sc * sc);
+    });
     const double d0 = sqrt(sm[0] * sh.inv_nn), d1 = sqrt(sm[1] * sh.inv_nn);
     const double h0 = (d0 < 1e-5 || d1 < 1e-5) ? 1e-6 : 0.01 * d0 / d1;
     const float c0 = (float)h0;
 #pragma unroll
     for (int q = 0; q < Q; ++q) v[q] = caxpy(c0, k1[q * NT], y[q * NT]);
     rhs(t + h0);
-    sm[0] = 0.0;
-#pragma unroll
-    for (int q = 0; q < Q; ++q)
-      if ((own >> q) & 1u) {
-        const double sc = o.atol + o.rtol * (double)cabsf(y[q * NT]), w = (strict >> q) & 1u ? 2.0 : 1.0;
-        const float2 f0 = k1[q * NT];
-        const double dx = (double)v[q].x - (double)f0.x, dy = (double)v[q].y - (double)f0.y;
-        sm[0] += w * (dx * dx + dy * dy) / (sc * sc);
-      }
-    sm[1] = 0.0;
-    block_sums(sm, sh, par);
-    const double d2 = sqrt(sm[0] * sh.inv_nn) / h0;
+    block_sums(s2, sh, par, [&](double (&e)[1], int r, int c) {
+      const int q = tile_of(r, c);
+      if (!((own >> q) & 1u)) return;
+      const double sc = o.atol + o.rtol * (double)cabsf(y[q * NT]), w = (strict >> q) & 1u ? 2.0 : 1.0;
+      const float2 f0 = k1[q * NT];
+      const double dx = (double)v[q].x - (double)f0.x, dy = (double)v[q].y - (double)f0.y;
+      e[0] += w * fma(dx, dx, dy * dy) / (sc * sc);
+    });
+    const double d2 = sqrt(s2[0] * sh.inv_nn) / h0;
     const double md = d1 > d2 ? d1 : d2;
     const double hh = md <= 1e-15 ? fmax(1e-6, h0 * 1e-3) : pow(0.01 / md, 0.25);
     dt_prop = fmin(100.0 * h0, hh);
@@ -677,33 +719,28 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
       copy(k[s], v);
     }
     // ---- embedded error, FP64 ----
-    double sm[1] = {0.0};
+    double sm[1];
     {
       const Tableau& tab = c_tab[o.method];
       double cb[7];
 #pragma unroll
       for (int j = 0; j < 7; ++j) cb[j] = h * tab.btilde[j];
-      int q = 0;
+      block_sums(sm, sh, par, [&](double (&e)[1], int r, int c) {
+        const int q = tile_of(r, c);
+        if (!((own >> q) & 1u)) return;
+        const float2 y1 = X[(ty + T * r) * LD + tx + T * c];
+        double ex = 0.0, ey = 0.0;
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int c = r; c < R; ++c, ++q) {
-          if ((own >> q) & 1u) {
-            const float2 y1 = X[(ty + T * r) * LD + tx + T * c];
-            double ex = 0.0, ey = 0.0;
-#pragma unroll
-            for (int j = 0; j < 7; ++j) {
-              const float2 kv = kval(j, q);
-              ex = fma(cb[j], (double)kv.x, ex);
-              ey = fma(cb[j], (double)kv.y, ey);
-            }
-            const float ya = cabsf(y[q * NT]), yb = cabsf(y1);
-            const double sc = o.atol + o.rtol * (double)(ya > yb ? ya : yb);
-            sm[0] += ratio(((strict >> q) & 1u ? 2.0 : 1.0) * (ex * ex + ey * ey), sc * sc);
-          }
+        for (int j = 0; j < 7; ++j) {
+          const float2 kv = kval(j, q);
+          ex = fma(cb[j], (double)kv.x, ex);
+          ey = fma(cb[j], (double)kv.y, ey);
         }
+        const float ya = cabsf(y[q * NT]), yb = cabsf(y1);
+        const double sc = o.atol + o.rtol * (double)(ya > yb ? ya : yb);
+        e[0] += ratio(((strict >> q) & 1u ? 2.0 : 1.0) * fma(ex, ex, ey * ey), sc * sc);
+      });
     }
-    block_sums(sm, sh, par);
     const double err = sqrt(sm[0] * sh.inv_nn);
     nsteps += 1;
     if (!(err < INFINITY)) {

@@ -148,3 +148,30 @@ def test_initial_state_is_the_given_one(cuda_device, n, batch):
     assert torch.equal(dq.mesolve(H, Ls, rho, [0.5]).states[:, 0], given.expand(batch, n, n))
     last = dq.mesolve(H, Ls, rho, [0.5], options=dq.Options(save_states=False))
     assert torch.equal(last.final_state.reshape(batch, n, n), given.expand(batch, n, n))
+
+
+@pytest.mark.parametrize('n', [1, 2, 7, 8, 9, 15, 16, 17, 23, 24, 25, 31, 32])
+@pytest.mark.parametrize('td', [False, True])
+def test_result_does_not_depend_on_the_batch(cuda_device, n, td):
+    """A large batch of n <= 32 instances takes another thread layout than a few: each instance
+    has the same bits -- states, expectation values, step counts -- as alone."""
+    H, Ls, rho, Es = _problem(n, n, 400, [(1, 0), (0,)])
+    ts = np.linspace(0.0, 0.6, 5)
+    rng = np.random.default_rng(n)
+    for _ in range(7):  # values near zero at t0: the order of their FP64 sums shows
+        X = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
+        Es.append((X - np.trace(X @ rho) / np.trace(rho) * np.eye(n)).astype(np.complex64))
+    vals = rng.normal(size=(400, 3))
+
+    def solve(b):
+        if not td:
+            return dq.mesolve(H[b], Ls, rho, ts, exp_ops=Es)
+        drive = dq.pwc([0.0, 0.2, 0.35, 0.6], vals[b], H[0])
+        return dq.mesolve(H[1] + drive, Ls, rho, ts, exp_ops=Es)
+
+    all_ = solve(slice(None))
+    for b in (0, 57, 399):
+        one = solve(b)
+        for k in ('nsteps', 'naccepted'):
+            assert int(getattr(one.infos, k)) == int(getattr(all_.infos, k)[b])
+        assert torch.equal(one.states, all_.states[b]) and torch.equal(one.expects, all_.expects[b])
