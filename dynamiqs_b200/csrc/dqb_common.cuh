@@ -20,6 +20,7 @@
 #include "../../include/dqb200.h"
 
 #include <cstring>
+#include "dqb_scalar.cuh"
 
 namespace dqb {
 
@@ -122,36 +123,6 @@ __host__ inline CtrlOpts make_ctrl(const dqb_ode_options& o) {
   c.save_states = o.save_states;
   c.check_hermitian = o.check_hermitian;
   return c;
-}
-
-// x / y in FP64 where y lies in FP32's normal range: FP32 reciprocal, two Newton steps
-// (relative error below 2^-50); the division otherwise (zero, infinite or NaN y included).
-__device__ __forceinline__ double ratio(double x, double y) {
-  const float f = (float)y;
-  if (f > 1e-30f && f < 1e30f) {
-    double r = (double)__frcp_rn(f);
-    r = fma(r, fma(-y, r, 1.0), r);
-    r = fma(r, fma(-y, r, 1.0), r);
-    return x * r;
-  }
-  return x / y;
-}
-
-// e^(-1/5) in FP64 for e in FP32's normal range: an FP32 start (relative error below 1e-5) and
-// two Newton steps x <- x + x (1 - e x^5) / 5, whose error is 3 times the square of the one
-// before; pow otherwise.  The controller computes it once per step, alone: pow's latency was
-// a fifth of a small instance's step (n = 64 kets, 1500 instances: SE_AFTER against 0.96 ms; one
-// n = 16 oscillator: OSC_AFTER against 0.39 ms).
-__device__ __forceinline__ double inverse_fifth_root(double e) {
-  const float f = (float)e;
-  if (!(f > 1e-30f && f < 1e30f)) return pow(e, -0.2);
-  double x = (double)exp2f(-0.2f * log2f(f));
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const double x2 = x * x;
-    x = fma(0.2 * x, fma(-e * x, x2 * x2, 1.0), x);
-  }
-  return x;
 }
 
 // Integral controller: factor = clip(safety * err^(-1/5), fmin, factormax) with

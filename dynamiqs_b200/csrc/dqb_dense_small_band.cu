@@ -738,7 +738,7 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
         }
         const float ya = cabsf(y[q * NT]), yb = cabsf(y1);
         const double sc = o.atol + o.rtol * (double)(ya > yb ? ya : yb);
-        e[0] += ratio(((strict >> q) & 1u ? 2.0 : 1.0) * fma(ex, ex, ey * ey), sc * sc);
+        e[0] += ((strict >> q) & 1u ? 2.0 : 1.0) * fma(ex, ex, ey * ey) / (sc * sc);
       });
     }
     const double err = sqrt(sm[0] * sh.inv_nn);
