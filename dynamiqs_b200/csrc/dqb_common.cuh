@@ -20,6 +20,7 @@
 #include "../../include/dqb200.h"
 
 #include <cstring>
+#include "dqb_per_device.cuh"
 #include "dqb_scalar.cuh"
 
 namespace dqb {
@@ -340,6 +341,21 @@ static __global__ void zero_words_kernel(unsigned int* p, int n) {
 template <class Kern>
 __host__ inline void prefer_max_shared(Kern kern) {
   cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+}
+
+// Raises a kernel's dynamic shared memory on the current device; whether it did.
+template <class Kern>
+__host__ inline bool raise_shared(Kern kern, int bytes) {
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess) return true;
+  cudaGetLastError();  // the launch that is not made reports it
+  return false;
+}
+
+// PerDevice::run on the current device.
+template <class F>
+__host__ inline bool on_this_device(PerDevice& p, F setup) {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess && p.run(dev, setup);
 }
 
 }  // namespace dqb

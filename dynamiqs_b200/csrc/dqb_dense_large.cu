@@ -1373,10 +1373,11 @@ void launch_hnh(cudaStream_t s, const big::Common& c, const LargeOps& d, int B, 
 
 using namespace dqb;
 
-// One-time: every kernel of this file asks for the same (largest) shared-memory carveout.
-static void init_carveouts() {
-  static std::once_flag once;
-  std::call_once(once, [] {
+// Once per device: every kernel of this file asks for the same (largest) shared-memory
+// carveout, the products for their dynamic shared memory.
+static bool init_kernels() {
+  static PerDevice once;
+  return on_this_device(once, [] {
     prefer_max_shared(big::setup_kernel);
     prefer_max_shared(big::load_rho0_kernel);
     prefer_max_shared(big::combine_kernel);
@@ -1411,9 +1412,10 @@ static void init_carveouts() {
     prefer_max_shared(choose_loop_kernel);
     prefer_max_shared(hnh_td_dense_kernel);
     prefer_max_shared(lt_td_dense_kernel);
-    auto dyn_attrs = [](auto kern, int smem) {
+    bool ok = true;
+    auto dyn_attrs = [&](auto kern, int smem) {
       prefer_max_shared(kern);
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      ok = raise_shared(kern, smem) && ok;
     };
     dyn_attrs(cgemm_kernel<2>, Tile<2>::kSmem);
     dyn_attrs(cgemm_kernel<3>, Tile<3>::kSmem);
@@ -1425,6 +1427,7 @@ static void init_carveouts() {
     dyn_attrs(tc_cgemm_kernel<DQB_PREC_TF32X3, 64>, tcg::Cfg<64>::kSmem);
     dyn_attrs(tc_cgemm_kernel<DQB_PREC_BF16X3, 64>, tcg::Cfg<64>::kSmem);
     dyn_attrs(tc_cgemm_kernel<DQB_PREC_TF32, 64>, tcg::Cfg<64>::kSmem);
+    return ok;
   });
 }
 
@@ -1435,7 +1438,7 @@ static void init_carveouts() {
 static int run_large(const big::Common& c, const LargeOps& d_in, cudaStream_t s, bool krylov,
                      const TdOps* td = nullptr, float2* hnh0 = nullptr, const JumpTd* jt = nullptr,
                      float2* Lt = nullptr) {
-  init_carveouts();
+  if (!init_kernels()) return DQB_ERR_CUDA;
   LargeOps d = d_in;
   JumpTd jtv;
   std::memset(&jtv, 0, sizeof(jtv));
@@ -1598,7 +1601,7 @@ extern "C" int dqb_lindblad_rhs_dense_large_prec(const dqb_dense_problem* p, int
   big::Common c;
   std::memset(&c, 0, sizeof(c));
   cudaStream_t s = (cudaStream_t)stream;
-  init_carveouts();
+  if (!init_kernels()) return DQB_ERR_CUDA;
   launch_hnh(s, c, d, (int)p->batch, 2);
   launch_rhs(s, c, d, (int)p->batch, 2, 0, 2, form, (const float2*)rho, (float2*)outp);
   return cudaGetLastError() == cudaSuccess ? DQB_OK : DQB_ERR_CUDA;

@@ -495,32 +495,38 @@ static size_t smem_for(int NP, int K) {
   }
 }
 
-// Occupancy of a persistent kernel for a dynamic shared-memory size.  The kernel's
-// dynamic shared-memory limit is raised once, to the device maximum, and never lowered:
-// the attribute is per-function state shared by every host thread, so per-call values
-// could race with another thread's launch.  Results are cached per (kernel, smem).
+// Occupancy of a persistent kernel for a dynamic shared-memory size, on the current device
+// (0 where its shared memory cannot be raised).  The kernel's dynamic shared-memory limit is
+// raised once per device, to the device maximum, and never lowered: the attribute is state
+// shared by every host thread, so per-call values could race with another thread's launch.
+// Results are kept per (device, kernel, smem).
 template <class Kern>
 static int resident_ctas(Kern kern, size_t smem) {
+  struct Entry {
+    int dev;
+    const void* fn;
+    size_t smem;
+    int per_sm;
+  };
   static std::mutex mu;
-  static std::vector<std::pair<const void*, size_t>> keys;  // (kernel, smem)
-  static std::vector<int> values;
-  static std::vector<const void*> raised;
+  static std::vector<Entry> entries;
+  static std::vector<std::pair<int, const void*>> raised;
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   const void* fn = (const void*)kern;
   std::lock_guard<std::mutex> lock(mu);
-  if (std::find(raised.begin(), raised.end(), fn) == raised.end()) {
+  if (std::find(raised.begin(), raised.end(), std::make_pair(dev, fn)) == raised.end()) {
     cudaFuncAttributes fa;
-    cudaFuncGetAttributes(&fa, kern);
-    const int limit = (int)max_optin_smem() - (int)fa.sharedSizeBytes;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return 0;
+    if (!raise_shared(kern, (int)max_optin_smem() - (int)fa.sharedSizeBytes)) return 0;
     prefer_max_shared(kern);
-    raised.push_back(fn);
+    raised.emplace_back(dev, fn);
   }
-  for (size_t i = 0; i < keys.size(); ++i)
-    if (keys[i].first == fn && keys[i].second == smem) return values[i];
+  for (const Entry& e : entries)
+    if (e.dev == dev && e.fn == fn && e.smem == smem) return e.per_sm;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSmallThreads, smem);
-  keys.emplace_back(fn, smem);
-  values.push_back(per_sm);
+  entries.push_back(Entry{dev, fn, smem, per_sm});
   return per_sm;
 }
 

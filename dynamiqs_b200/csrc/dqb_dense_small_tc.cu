@@ -536,13 +536,13 @@ __global__ void bounded_wait_probe_kernel(unsigned long long limit_ns, int* out)
   out[1] = (int)((tc::globaltimer_ns() - t0) / 1000ull);
 }
 
-static void raise_smem_limit_once() {
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaFuncSetAttribute(mesolve_small_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, stc::smem_bytes(2));
-    cudaFuncSetAttribute(rhs_small_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, stc::smem_bytes(2));
+static bool init_kernels() {  // once per device
+  static PerDevice once;
+  return on_this_device(once, [] {
     prefer_max_shared(mesolve_small_tc_kernel);
     prefer_max_shared(rhs_small_tc_kernel);
+    return raise_shared(mesolve_small_tc_kernel, stc::smem_bytes(2)) &&
+           raise_shared(rhs_small_tc_kernel, stc::smem_bytes(2));
   });
 }
 
@@ -555,7 +555,7 @@ bool small_tc_applies(int n, int K, int form) {
 // Launch the persistent tensor-core kernel: one CTA per SM (at most `batch`), the work
 // counter at `counter` (zeroed by the caller) and the CTAs' slots at `slots`.
 int small_tc_launch(const DenseSmallArgs& a, int max_grid, cudaStream_t s) {
-  raise_smem_limit_once();
+  if (!init_kernels()) return DQB_ERR_CUDA;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -569,7 +569,7 @@ int small_tc_launch(const DenseSmallArgs& a, int max_grid, cudaStream_t s) {
 // One right-hand side per instance on the tensor cores; `scratch` holds batch x 64 x 64
 // complex64.
 int small_tc_rhs(const DenseSmallArgs& a, const float2* rho, float2* out, float2* scratch, cudaStream_t s) {
-  raise_smem_limit_once();
+  if (!init_kernels()) return DQB_ERR_CUDA;
   DenseSmallArgs b = a;
   b.slots = scratch;
   rhs_small_tc_kernel<<<(unsigned)a.batch, kSmallThreads, stc::smem_bytes(a.K), s>>>(b, rho, out);

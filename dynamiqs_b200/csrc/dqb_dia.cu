@@ -1386,10 +1386,11 @@ struct LaunchKey {
 
 using namespace dqb;
 
-// One-time: every kernel of this file asks for the same (largest) shared-memory carveout.
-static void init_carveouts() {
-  static std::once_flag once;
-  std::call_once(once, [] {
+// Once per device: every kernel of this file asks for the same (largest) shared-memory
+// carveout, the stencils for their dynamic shared memory.
+static bool init_kernels() {
+  static PerDevice once;
+  return on_this_device(once, [] {
     prefer_max_shared(big::setup_kernel);
     prefer_max_shared(big::load_rho0_kernel);
     prefer_max_shared(big::combine_kernel);
@@ -1421,16 +1422,14 @@ static void init_carveouts() {
     prefer_max_shared(rhs_dia_tiled_kernel<4>);
     prefer_max_shared(rhs_dia_tiled_kernel<8>);
     prefer_max_shared(rhs_dia_tiled_kernel<16>);
-    prefer_max_shared(rhs_dia_staged_kernel<8>);
-    prefer_max_shared(rhs_dia_staged_kernel<16>);
-    auto herm_attr = [](auto kern) {
+    bool ok = true;
+    auto herm_attr = [&](auto kern) {
       prefer_max_shared(kern);
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           16 * (kRhsCols * 4 + 1) * (int)sizeof(float2));
+      ok = raise_shared(kern, 16 * (kRhsCols * 4 + 1) * (int)sizeof(float2)) && ok;
     };
-    auto bulk_attr = [](auto kern) {
+    auto bulk_attr = [&](auto kern) {
       prefer_max_shared(kern);
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxSmem);
+      ok = raise_shared(kern, (int)kStageMaxSmem) && ok;
     };
     bulk_attr(rhs_dia_bulk_kernel<4, 4, 2>);
     bulk_attr(rhs_dia_bulk_kernel<4, 4, 4>);
@@ -1444,8 +1443,9 @@ static void init_carveouts() {
     herm_attr(rhs_dia_wide_kernel<16, 4, 4, 4, true>);
     herm_attr(rhs_dia_wide_kernel<16, 8, 2, 4, true>);
     herm_attr(rhs_dia_wide_kernel<16, 8, 4, 4, true>);
-    cudaFuncSetAttribute(rhs_dia_staged_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxSmem);
-    cudaFuncSetAttribute(rhs_dia_staged_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageMaxSmem);
+    bulk_attr(rhs_dia_staged_kernel<8>);
+    bulk_attr(rhs_dia_staged_kernel<16>);
+    return ok;
   });
 }
 
@@ -1476,7 +1476,7 @@ extern "C" int dqb_lindblad_rhs_dia_tiled(const dqb_dia_problem* p, int32_t form
   if (!workspace || workspace_bytes < need) return DQB_ERR_WORKSPACE_TOO_SMALL;
   d.hnh = (float2*)workspace;
   cudaStream_t s = (cudaStream_t)stream;
-  init_carveouts();
+  if (!init_kernels()) return DQB_ERR_CUDA;
   hnh_dia_kernel<<<dim3((p->n + 255) / 256, (unsigned)p->batch), 256, 0, s>>>(d, (int)p->batch);
   big::Common c;
   std::memset(&c, 0, sizeof(c));
@@ -1574,7 +1574,7 @@ static int solve_dia(const dqb_dia_problem* p, const dqb_td_hamiltonian* tdh, co
   const int T = big::kElemThreads;
 
   // ---- set-up and starting step (outside the graph) ----------------------------------
-  init_carveouts();
+  if (!init_kernels()) return DQB_ERR_CUDA;
   big::setup_kernel<<<gi, 128, 0, s>>>(c);
   if (!jt.on) {  // (with time-dependent jump operators every Hnh is formed at its time)
     DiaOps d0 = d;  // the constant Hnh: into hnh, or into hnh0 when H depends on time

@@ -262,15 +262,14 @@ void launch_save(cudaStream_t s, const big::Common& c, int mode) {
                    (size_t)c.n * sizeof(float2), s>>>(c, mode);
 }
 
-void init_attrs() {
-  static std::once_flag once;
-  std::call_once(once, [] {
+bool init_kernels() {  // once per device
+  static PerDevice once;
+  return on_this_device(once, [] {
     prefer_max_shared(se_rhs_dense_kernel);
     prefer_max_shared(se_save_kernel);
     prefer_max_shared(se_h_td_kernel);
-    cudaFuncSetAttribute(se_rhs_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kSeMaxN * (int)sizeof(float2));
-    cudaFuncSetAttribute(se_save_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSeMaxN * (int)sizeof(float2));
+    return raise_shared(se_rhs_dense_kernel, kSeMaxN * (int)sizeof(float2)) &&
+           raise_shared(se_save_kernel, kSeMaxN * (int)sizeof(float2));
   });
 }
 
@@ -334,7 +333,7 @@ int run(const SeOps& d0, int nE, int ntsave, long long B, const void* psi0, cons
     c.jump_ts = tdh->jump_ts;
   }
 
-  init_attrs();
+  if (!init_kernels()) return DQB_ERR_CUDA;
   int grid_e = (int)std::min<long long>((c.nn + big::kElemThreads - 1) / big::kElemThreads, 1184);
   if (grid_e < 1) grid_e = 1;
   const dim3 ge(grid_e, c.B);
