@@ -681,9 +681,10 @@ class MESolveB200Integrator:
             tr = torch.empty(states.shape[:-2], dtype=torch.complex128, device=states.device)
             size = lib.dqb_state_checks_workspace_size(n, count)
             ws = torch.empty(size, dtype=torch.uint8, device=states.device)
-            rc = lib.dqb_state_checks(st.data_ptr(), n, count, herm.data_ptr(), tr.data_ptr(),
-                                      ws.data_ptr(), size,
-                                      torch.cuda.current_stream(states.device).cuda_stream)
+            with torch.cuda.device(states.device):  # (the caller may have made another current)
+                rc = lib.dqb_state_checks(st.data_ptr(), n, count, herm.data_ptr(), tr.data_ptr(),
+                                          ws.data_ptr(), size,
+                                          torch.cuda.current_stream(states.device).cuda_stream)
             _lib.check(rc, 'dqb_state_checks')
         return {'trace': tr if trace is None else trace, 'hermiticity': herm}
 

@@ -234,3 +234,36 @@ def test_upload_is_the_array(cuda_device, nbytes):
         assert np.array_equal(out['a'].cpu().numpy(), want)
         assert np.array_equal(out['ro'].cpu().numpy(), ro.astype(np.complex64))
         assert out['i'].dtype == torch.int32 and out['i'].tolist() == list(range(7))
+
+
+def test_result_checks_run_on_the_states_device(monkeypatch):
+    """The checks of the saved states are launched with the states' device current, whatever
+    device the caller has made current since the solve."""
+    import contextlib
+    import types
+
+    import torch
+
+    from dynamiqs_b200.mesolve import MESolveB200Integrator
+
+    current = []
+
+    @contextlib.contextmanager
+    def device(d):
+        current.append(d)
+        yield
+        current.pop()
+
+    def checks(*args):
+        launched.append(list(current))
+        return 0
+
+    launched = []
+    lib = types.SimpleNamespace(dqb_state_checks=checks, dqb_state_checks_workspace_size=lambda n, count: 8)
+    monkeypatch.setattr(_lib, 'load', lambda: lib)
+    monkeypatch.setattr(torch.cuda, 'device', device)
+    monkeypatch.setattr(torch.cuda, 'current_stream', lambda d=None: types.SimpleNamespace(cuda_stream=0))
+    states = torch.zeros((2, 3, 4, 4), dtype=torch.complex64)
+    out = MESolveB200Integrator._checks(None, states, None)
+    assert launched == [[states.device]] and current == []
+    assert out['trace'].shape == out['hermiticity'].shape == (2, 3)
