@@ -28,6 +28,7 @@ PACK_BYTES = 1 << 18  # arrays up to this size are packed together
 RING_BYTES = 24 << 20  # arrays from this size on go through the ring
 SLOT_BYTES = 2 << 20
 SLOTS = 12
+AHEAD = 6  # slots being filled; the copies of the others are in flight
 THREADS = 4
 _ALIGN = 256
 
@@ -56,12 +57,6 @@ def _host_array(x, dtype):
     return a
 
 
-def _fill(slot, chunk, done) -> None:
-    if done is not None:
-        done.synchronize()  # the slot's previous contents have left
-    np.copyto(slot, chunk)
-
-
 def _ring_copy(dst, a) -> None:
     """The bytes of ``a`` into the device tensor ``dst``, on the current stream."""
     import torch
@@ -76,18 +71,23 @@ def _ring_copy(dst, a) -> None:
     def fill(i):
         o, s = chunks[i], i % SLOTS * SLOT_BYTES
         m = min(SLOT_BYTES, src.size - o)
-        return submit(_fill, host[s:s + m], src[o:o + m], done[i % SLOTS])
+        # This thread waits until the slot's previous contents have left: the threads of the
+        # pool serve every caller, and one that waited for a busy stream would hold up uploads
+        # to others.
+        if done[i % SLOTS] is not None:
+            done[i % SLOTS].synchronize()
+        return submit(np.copyto, host[s:s + m], src[o:o + m])
 
     submit = _pool().submit
-    filled = [fill(i) for i in range(min(SLOTS, len(chunks)))]
+    filled = [fill(i) for i in range(min(AHEAD, len(chunks)))]
     for i, o in enumerate(chunks):
         filled[i].result()
         s, m = i % SLOTS * SLOT_BYTES, min(SLOT_BYTES, src.size - o)
         out[o:o + m].copy_(ring[s:s + m], non_blocking=True)
         done[i % SLOTS] = torch.cuda.Event()
         done[i % SLOTS].record()
-        if i + SLOTS < len(chunks):
-            filled.append(fill(i + SLOTS))
+        if i + AHEAD < len(chunks):
+            filled.append(fill(i + AHEAD))
 
 
 def to_device(items: dict, device) -> dict:

@@ -1,6 +1,8 @@
 """Host-side logic of the drop-in API: argument checks with the reference's messages,
 batching plans (cartesian and flat, mesolve.py:307-336) and the no-fallback rule."""
 
+import time
+
 import numpy as np
 import pytest
 
@@ -267,3 +269,38 @@ def test_result_checks_run_on_the_states_device(monkeypatch):
     out = MESolveB200Integrator._checks(None, states, None)
     assert launched == [[states.device]] and current == []
     assert out['trace'].shape == out['hermiticity'].shape == (2, 3)
+
+
+@pytest.mark.gpu
+def test_upload_is_not_held_up_by_another_stream(cuda_device):
+    """An upload on a busy stream, more than the ring's slots long, waits for that stream; one
+    on an idle stream in another thread meanwhile does not."""
+    import threading
+
+    import torch
+
+    from dynamiqs_b200.upload import to_device
+
+    big = np.ones((80 << 20) // 8, np.complex64)
+    small = np.ones((32 << 20) // 8, np.complex64)
+    to_device({'x': (big, torch.complex64)}, cuda_device)  # the page-locked blocks, the threads
+    busy, idle = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(3_000_000_000)  # about 1.5 s, then it ends
+        end = torch.cuda.Event()
+        end.record()
+
+    def upload():
+        with torch.cuda.stream(busy):
+            to_device({'x': (big, torch.complex64)}, cuda_device)
+
+    other = threading.Thread(target=upload)
+    other.start()
+    time.sleep(0.3)  # the first upload fills its ring and waits
+    with torch.cuda.stream(idle):
+        out = to_device({'x': (small, torch.complex64)}, cuda_device)['x']
+        idle.synchronize()
+        done_first = not end.query()
+    other.join()
+    assert done_first and bool((out == 1).all())
