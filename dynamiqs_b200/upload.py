@@ -18,7 +18,7 @@ exit.
 from __future__ import annotations
 
 import threading
-from concurrent.futures import ThreadPoolExecutor
+from concurrent.futures import Future, ThreadPoolExecutor
 
 import numpy as np
 
@@ -42,6 +42,17 @@ def _pool() -> ThreadPoolExecutor:
         if _POOL is None:
             _POOL = ThreadPoolExecutor(THREADS, thread_name_prefix='dqb-upload')
         return _POOL
+
+
+def _submit(fn, *args) -> Future:
+    """``fn(*args)`` on a thread of the pool, or here where none can be had (the interpreter is
+    exiting, or the process is out of threads)."""
+    try:
+        return _pool().submit(fn, *args)
+    except RuntimeError:
+        done = Future()
+        done.set_result(fn(*args))
+        return done
 
 
 def _host_array(x, dtype):
@@ -76,9 +87,8 @@ def _ring_copy(dst, a) -> None:
         # to others.
         if done[i % SLOTS] is not None:
             done[i % SLOTS].synchronize()
-        return submit(np.copyto, host[s:s + m], src[o:o + m])
+        return _submit(np.copyto, host[s:s + m], src[o:o + m])
 
-    submit = _pool().submit
     filled = [fill(i) for i in range(min(AHEAD, len(chunks)))]
     for i, o in enumerate(chunks):
         filled[i].result()

@@ -304,3 +304,27 @@ def test_upload_is_not_held_up_by_another_stream(cuda_device):
         done_first = not end.query()
     other.join()
     assert done_first and bool((out == 1).all())
+
+
+def test_upload_copies_without_its_threads():
+    """While the interpreter exits no thread can be started: the slots are then filled by the
+    caller."""
+    import os
+    import subprocess
+    import sys
+
+    program = """
+import atexit
+import numpy as np
+from dynamiqs_b200 import upload
+
+def late():
+    a = np.zeros(5)
+    upload._submit(np.copyto, a, np.arange(5.0)).result()
+    print(a.tolist())
+
+atexit.register(late)
+"""
+    out = subprocess.run([sys.executable, '-c', program], capture_output=True, text=True, timeout=120,
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert out.stdout.strip() == '[0.0, 1.0, 2.0, 3.0, 4.0]', out.stderr
