@@ -282,6 +282,13 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
   constexpr int NP = G::NP, LD = G::LD, NT = G::NT, Q = G::Q;
   constexpr bool kTd = FEAT == 1, kTape = FEAT == 2;
   constexpr int kStep = Q <= 3 && !kTd ? 4 : 1;
+  // Diagonals of a jump operator from which the right-hand side multiplies it in two steps (V
+  // below) and not term by term, and diagonals per pass there.  Measured at n = 8 and 16, one
+  // instance, four diagonals: 63 and 72 us in two steps, 99 and 118 term by term, 70 and 92
+  // with the products of full matrices; n = 32: 107, 144 and 176.  With T = 8 two steps pay
+  // later (their transposed reads of V conflict on banks): n = 4 with full jumps, 2000
+  // instances, 275 against 823 us, but three diagonals the same either way.
+  constexpr int kFactor = T == 16 ? (R == 1 ? 2 : 3) : 4, kGroup = T == 16 && R == 1 && !kTd ? 4 : 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tx = tid % T, ty = tid / T;
   const InstView& a = sh.v;
@@ -299,9 +306,24 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
   const int K = a.K;
   if (K > kMaxK) return false;
   for (int e = tid; e < (1 + kMaxK + kMaxM) * 4; e += NT) (&ls.mask[0][0])[e] = 0u;
-  // the nonzeros of one row lie on as many diagonals: full matrices are told by one row
-  const float2 mid = tid < n ? __ldg(a.H + n / 2 * n + tid) : make_float2(0.f, 0.f);
-  if (__syncthreads_count(mid.x != 0.f || mid.y != 0.f) > kMaxH) return false;
+  // Full matrices are told by their first and last rows: the nonzeros of the two lie on
+  // different diagonals but for the main one, which both may have.  (A middle row alone tells
+  // them only beyond 8 columns, and one instance of n = 8 spent 11 us on its lists.)
+  unsigned ends = 0;  // bit m: a nonzero of operator m (H, the jumps) at the thread's place
+  if (tid < 2 * n) {
+    const long long at = tid < n ? tid : (long long)n * n - 2 * n + tid;
+    float2 e = __ldg(a.H + at);
+    ends = e.x != 0.f || e.y != 0.f;
+#pragma unroll 1
+    for (int k = 0; k < K; ++k) {
+      e = __ldg(a.L + (long long)k * n * n + at);
+      if (e.x != 0.f || e.y != 0.f) ends |= 2u << k;
+    }
+  }
+  if (__syncthreads_count(ends & 1u) > kMaxH + 1) return false;
+  int jumps = 0;
+  for (int k = 0; k < K; ++k) jumps += __syncthreads_count(ends >> (k + 1) & 1u);
+  if (jumps > kMaxL + K) return false;
   scan_diagonals<NT>(a.H, n, ls.mask[0]);
   for (int k = 0; k < K; ++k) scan_diagonals<NT>(a.L + (long long)k * n * n, n, ls.mask[1 + k]);
   for (int m = 0; m < M; ++m) scan_diagonals<NT>(td->ops + (long long)m * n * n, n, ls.mask[1 + kMaxK + m]);
@@ -569,6 +591,58 @@ __device__ bool solve(const CtrlOpts& o, const TdArgs* td, Shared<T, R>& sh, flo
               S[q] = cfma(u, cr[r], S[q]);
             }
           }
+        continue;
+      }
+      if (p1 - p0 >= kFactor) {
+        // Many diagonals: V = X L^+ first, whole, in the buffer that the previous right-hand side
+        // has left, so that each of the two sums below runs over the diagonals once.  By X's
+        // hermiticity V[i + p][j] = conj((L X)[j][i + p]) and conj(V[j + t][i]) = (L X)[i][j + t].
+        float2* V = Xb[xb ^ 1];
+#pragma unroll 1
+        for (int r = 0; r < R; ++r) {
+          float2 u[R];
+#pragma unroll
+          for (int c = 0; c < R; ++c) u[c] = make_float2(0.f, 0.f);
+          const int i = ty + T * r;
+#pragma unroll 1
+          for (int t0 = p0; t0 < p1; t0 += kGroup) {
+#pragma unroll
+            for (int tt = 0; tt < kGroup; ++tt) {
+              const int t = min(t0 + tt, kMaxL - 1), off = offset_of(loffs, t);
+#pragma unroll
+              for (int c = 0; c < R; ++c) {
+                const int j = tx + T * c;
+                float2 w = cconj(ld[t * NP + j]);
+                if (tt > 0 && t0 + tt >= p1) w = make_float2(0.f, 0.f);
+                u[c] = cfma(w, X[i * LD + min(max(j + off, 0), NP - 1)], u[c]);
+              }
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < R; ++c) V[i * LD + tx + T * c] = make_float2(0.5f * u[c].x, 0.5f * u[c].y);
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int t0 = p0; t0 < p1; t0 += kGroup) {
+#pragma unroll
+          for (int tt = 0; tt < kGroup; ++tt) {
+            const int t = min(t0 + tt, kMaxL - 1), off = offset_of(loffs, t);
+            coefs(ld + t * NP, ld + t * NP);
+            displaced(off, off);
+            const bool in = tt == 0 || t0 + tt < p1;
+            int q = 0;
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+              for (int c = r; c < R; ++c, ++q) {
+                float2& dst = G::diag_block(r, c) ? B[q] : S[q];
+                const float2 none = make_float2(0.f, 0.f);
+                dst = cfma(V[xr[r] + tx + T * c], in ? cr[r] : none, dst);
+                if (G::diag_block(r, c)) A[q] = cfma(cconj(V[xc[c] * LD + ty + T * r]), in ? cc[c] : none, A[q]);
+              }
+          }
+        }
+        __syncthreads();  // V has been read
         continue;
       }
 #pragma unroll 1

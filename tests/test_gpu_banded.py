@@ -175,3 +175,21 @@ def test_result_does_not_depend_on_the_batch(cuda_device, n, td):
         for k in ('nsteps', 'naccepted'):
             assert int(getattr(one.infos, k)) == int(getattr(all_.infos, k)[b])
         assert torch.equal(one.states, all_.states[b]) and torch.equal(one.expects, all_.expects[b])
+
+
+@pytest.mark.parametrize('n, batch', [(n, 2) for n in (5, 8, 16, 17, 32, 33, 48, 49, 64)]
+                         + [(n, 400) for n in (5, 8, 9, 16, 17, 24, 25, 32)])
+@pytest.mark.parametrize('jumps', [[(-1, 0, 1), (0, 2)], [(-1, 0, 1, 2), (-2, -1, 0, 1)]])
+def test_jumps_of_many_diagonals(cuda_device, n, batch, jumps):
+    """Jump operators multiplied in two steps, in both thread layouts, constant and in a
+    time-dependent problem."""
+    H, Ls, rho, Es = _problem(n, n, batch, jumps)
+    ts = [0.0, 0.1, 0.3]
+    _agree(dq.mesolve(H, Ls, rho, ts, exp_ops=Es), dq.mesolve(H + np.complex64(1e-25), Ls, rho, ts, exp_ops=Es))
+    # (a smooth drive: with a jump in time, a stage whose time rounds onto the jump takes a step's
+    # decision by the last bit of that step)
+    wave = dq.Wave(amplitude=0.7, omega=3.0)
+    rhos = np.stack([rho] * batch)
+    a, b = (dq.mesolve(h + dq.modulated(wave, H[1]), Ls, rhos, ts, exp_ops=Es)
+            for h in (H[0], H[0] + np.complex64(1e-25)))
+    _agree(a, b)
