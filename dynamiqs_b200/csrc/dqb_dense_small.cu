@@ -218,7 +218,18 @@ __device__ void rhs(const float2* sH, const float2* sL, const float2* sX, float2
 // Used where the state is not hermitian by construction -- the standard form and the adjoint --;
 // the hermitian form's banded instances have a kernel of their own (dqb_dense_small_band.cu).
 
-constexpr int kBandDiags = 8;  // diagonals of Hnh, and of the jumps together
+constexpr int kBandDiags = 8;  // diagonals of Hnh, and of each jump (what the tables hold)
+
+// Whether the standard form of an instance with `diags` nonzero diagonals (Hnh and the jumps
+// together) takes the sums over diagonals: a diagonal costs its address arithmetic, a product
+// n steps of the inner loop, so with 16 x 16 tiles few columns are multiplied sooner.  The
+// line lies where the two measured the same (2000 instances, no jump: n = 4 between 3 and 6
+// diagonals, n = 8 between 3 and 6, n = 16 at 7; n = 8, 8 diagonals: 585 us against 482 with
+// products; a jump operator moves it by the products it saves).  With larger tiles eight
+// diagonals are always the faster ones (n = 24: 920 against 1046 us).
+__device__ __forceinline__ bool stencil_pays(int NP, int n, int K, int diags) {
+  return NP > 16 || diags <= 3 + n / 4 + K * (2 + n / 8);
+}
 
 struct Bands {
   unsigned mask[3][4];  // Hnh, L_1, L_2: bit j - i + 63
@@ -363,8 +374,16 @@ struct SimtEngine {
       __syncthreads();
     }
     if constexpr (!kJumps) {
-      if (form == DQB_FORM_STANDARD && K <= 2) find_bands<NP>(*bl, sH, sL, K);
-      else if (threadIdx.x == 0) bl->ok = 0;
+      if (form == DQB_FORM_STANDARD && K <= 2) {
+        find_bands<NP>(*bl, sH, sL, K);
+        if (threadIdx.x == 0 && bl->ok) {
+          int diags = bl->nh;
+          for (int k = 0; k < K; ++k) diags += bl->nl[k];
+          bl->ok = stencil_pays(NP, n, K, diags);
+        }
+      } else if (threadIdx.x == 0) {
+        bl->ok = 0;
+      }
       __syncthreads();
     }
   }

@@ -102,3 +102,12 @@ def test_adjoint_with_eight_diagonals(cuda_device, n):
 
     for a, b in zip(grads(H), grads(H + np.complex64(1e-25))):
         assert (a - b).abs().max() <= 64 * 2 ** -24 * b.abs().max()
+
+
+@pytest.mark.parametrize('n', [2, 4, 8, 16])
+@pytest.mark.parametrize('offsets', [(0, 1), (0, 1, 2), (1, 2, 3), (0, 1, 2, 3), (1, 2, 3, 4)])
+@pytest.mark.parametrize('jumps', [[], [(1,)], [(0, 1), (-1,)]])
+def test_standard_form_small(cuda_device, n, offsets, jumps):  # either side of stencil_pays
+    rng = np.random.default_rng(n)
+    _check(_band(rng, n, offsets, 0.3, True), [_band(rng, n, off, 0.2) for off in jumps], _ket(rng, n),
+           _band(rng, n, (0, 1), 0.5, True), assume_hermitian=False)
