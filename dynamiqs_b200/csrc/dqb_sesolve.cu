@@ -14,8 +14,8 @@
 //     Hamiltonians have), listed on the device; the product is a stencil of those
 //     diagonals, so a step is short and one warp takes an instance, lane l holding the
 //     entries l + 32 r.  Its small shared memory (diagonals and stage input) lets every warp
-//     slot of the SM hold an instance.  Instances with a full H are marked in their step
-//     counts and left to
+//     slot of the SM hold an instance.  Instances with a full H of more than 32 rows are
+//     marked in their step counts and left to
 //   * full_kernel: one CTA per instance, one thread per row, the operator in shared memory
 //     (rows at an odd stride, so that the lanes' reads down a column are free of bank
 //     conflicts) or, beyond 128 rows, read from global memory along its columns.
@@ -371,9 +371,18 @@ __device__ __forceinline__ void load_tableau(double* a21, int method) {
 }
 
 // One warp per CTA and instance; n <= 32 R.  Shared memory: kMaxH diagonals, two x buffers.
-template <int R>
-__global__ void __launch_bounds__(32) band_kernel(Args a) {
+// kFull (R = 1): a full H is solved here, too, its operator in dynamic shared memory, and
+// full_kernel is not launched: up to 32 rows a warp has a row per lane and the operator costs
+// few resident warps.  One instance of n = 5, full H: 43 us against 52 with the second launch
+// (40 in a kernel with a 33 KB tile per warp); n = 32: 67 and 79; 20000 of n = 16: 436 and
+// 535, banded 243 and 261.
+constexpr int kFullMaxN = 32;
+
+template <int R, bool kFull>
+__global__ void __launch_bounds__(32, kFull ? 20 : (R == 2 ? 16 : 12)) band_kernel(Args a) {
+  static_assert(!kFull || R == 1, "one row per lane");
   constexpr int NP = 32 * R;
+  extern __shared__ float4 se_smem[];
   __shared__ float2 sd[kMaxH * NP];
   __shared__ float2 sx[2 * NP];
   __shared__ double a21[21];
@@ -397,57 +406,66 @@ __global__ void __launch_bounds__(32) band_kernel(Args a) {
       const float2 e = lane + 32 * r < n ? __ldg(H + (long long)(n / 2) * n + lane + 32 * r) : make_float2(0.f, 0.f);
       mid += __popc(__ballot_sync(0xffffffffu, e.x != 0.f || e.y != 0.f));
     }
-    if (mid > kMaxH) {
-      if (lane == 0) a.infos[inst * 3] = kPending;
-      continue;
-    }
-    // nonzero diagonals (bit j - i + n - 1)
-    constexpr int U = 8 / R;  // rows in flight
-    for (int i0 = 0; i0 < n; i0 += U) {
-      float2 e[U][R];
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int i = i0 + u, j = lane + 32 * r;
-          e[u][r] = (i < n && j < n) ? __ldg(H + (long long)i * n + j) : make_float2(0.f, 0.f);
-        }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-          if (e[u][r].x != 0.f || e[u][r].y != 0.f) {
-            const int b = lane + 32 * r - (i0 + u) + n - 1;
-            if (!(*(volatile unsigned*)&mask[b >> 5] >> (b & 31) & 1u)) atomicOr(&mask[b >> 5], 1u << (b & 31));
-          }
-    }
-    for (int e = lane; e < kMaxH * NP; e += 32) sd[e] = make_float2(0.f, 0.f);
-    __syncwarp();
     BandOp A;
     A.d = sd;
     A.ld = NP;
     A.nd = 0;
     A.off = A.off_hi = 0;
-    bool ok = true;
-    for (int w = 0; w < 8; ++w)
-      for (unsigned x = mask[w]; x; x &= x - 1) {
-        if (A.nd == kMaxH) {
-          ok = false;
-          break;
-        }
-        const int off = 32 * w + __ffs((int)x) - 1 - (n - 1);
-        const unsigned long long f = (unsigned long long)(off & 0xffff) << (16 * (A.nd & 3));
-        if (A.nd < 4) A.off |= f;
-        else A.off_hi |= f;
-        for (int i = lane; i < NP; i += 32) {
-          const int j = i + off;
-          sd[A.nd * NP + i] = (i < n && j >= 0 && j < n) ? __ldg(H + (long long)i * n + j) : make_float2(0.f, 0.f);
-        }
-        ++A.nd;
+    bool ok = mid <= kMaxH;
+    if (ok) {
+      // nonzero diagonals (bit j - i + n - 1)
+      constexpr int U = 8 / R;  // rows in flight
+      for (int i0 = 0; i0 < n; i0 += U) {
+        float2 e[U][R];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const int i = i0 + u, j = lane + 32 * r;
+            e[u][r] = (i < n && j < n) ? __ldg(H + (long long)i * n + j) : make_float2(0.f, 0.f);
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            if (e[u][r].x != 0.f || e[u][r].y != 0.f) {
+              const int b = lane + 32 * r - (i0 + u) + n - 1;
+              if (!(*(volatile unsigned*)&mask[b >> 5] >> (b & 31) & 1u)) atomicOr(&mask[b >> 5], 1u << (b & 31));
+            }
       }
-    __syncwarp();
+      for (int e = lane; e < kMaxH * NP; e += 32) sd[e] = make_float2(0.f, 0.f);
+      __syncwarp();
+      for (int w = 0; w < 8; ++w)
+        for (unsigned x = mask[w]; x; x &= x - 1) {
+          if (A.nd == kMaxH) {
+            ok = false;
+            break;
+          }
+          const int off = 32 * w + __ffs((int)x) - 1 - (n - 1);
+          const unsigned long long f = (unsigned long long)(off & 0xffff) << (16 * (A.nd & 3));
+          if (A.nd < 4) A.off |= f;
+          else A.off_hi |= f;
+          for (int i = lane; i < NP; i += 32) {
+            const int j = i + off;
+            sd[A.nd * NP + i] = (i < n && j >= 0 && j < n) ? __ldg(H + (long long)i * n + j) : make_float2(0.f, 0.f);
+          }
+          ++A.nd;
+        }
+      __syncwarp();
+    }
     if (!ok) {
-      if (lane == 0) a.infos[inst * 3] = kPending;
+      if constexpr (kFull) {
+        const int ld = n | 1;
+        float2* sA = reinterpret_cast<float2*>(se_smem);
+        for (int p = 0; p < n; ++p)
+          if (lane < n) sA[p * ld + lane] = __ldg(H + p * n + lane);
+        __syncwarp();
+        const FullOp F{sA, nullptr, ld};
+        Team<1, false> tm{nullptr, 0};
+        solve_instance(a, inst, F, tm, sx, NP, cf, a21);
+      } else if (lane == 0) {
+        a.infos[inst * 3] = kPending;
+      }
       continue;
     }
     Team<R, false> tm{nullptr, 0};
@@ -610,10 +628,11 @@ static int run(se::Args& a, const dqb_dense_problem* p, const dqb_ode_options* o
   a.o = make_ctrl(*o);
   const int n = p->n, threads = 32 * ((n + 31) / 32);
   zero_words_kernel<<<1, 64, 0, s>>>((unsigned int*)workspace, 64);
+  if (a.mode == se::kSchrodinger && n <= se::kFullMaxN)
+    return se::launch<se::band_kernel<1, true>>(a, 32, (size_t)n * (n | 1) * sizeof(float2), s);
   if (a.mode == se::kSchrodinger) {  // the banded instances first; the others are marked
-    const int rc = n <= 32 ? se::launch<se::band_kernel<1>>(a, 32, 0, s)
-                           : (n <= 64 ? se::launch<se::band_kernel<2>>(a, 32, 0, s)
-                                      : se::launch<se::band_kernel<4>>(a, 32, 0, s));
+    const int rc = n <= 64 ? se::launch<se::band_kernel<2, false>>(a, 32, 0, s)
+                           : se::launch<se::band_kernel<4, false>>(a, 32, 0, s);
     if (rc) return rc;
     a.counter += 1;
     a.pending_only = 1;

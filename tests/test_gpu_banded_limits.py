@@ -111,3 +111,18 @@ def test_standard_form_small(cuda_device, n, offsets, jumps):  # either side of 
     rng = np.random.default_rng(n)
     _check(_band(rng, n, offsets, 0.3, True), [_band(rng, n, off, 0.2) for off in jumps], _ket(rng, n),
            _band(rng, n, (0, 1), 0.5, True), assume_hermitian=False)
+
+
+@pytest.mark.parametrize('n', [5, 16, 31, 32, 33])
+def test_sesolve_full_and_banded(cuda_device, n):
+    """One launch for both up to 32 rows, two beyond: each instance of a mixed batch gives the
+    bits that it gives alone, and the full ones the oracle's states."""
+    rng = np.random.default_rng(n)
+    H = np.stack([_band(rng, n, (0, 1) if b % 2 else range(n), 0.3, True) for b in range(6)])
+    psi, E = _ket(rng, n), _band(rng, n, (0, 1), 0.5, True)
+    res = dq.sesolve(H, psi, TS, exp_ops=[E])
+    for b in range(6):
+        one = dq.sesolve(H[b], psi, TS, exp_ops=[E])
+        assert torch.equal(one.states, res.states[b]) and torch.equal(one.expects, res.expects[b])
+        ref = np.stack(oracle_sesolve(H[b], psi, TS, rtol=1e-6, atol=1e-6, save_fn=lambda y: y).ysave)
+        assert np.linalg.norm(one.states.cpu().numpy() - ref, axis=(-2, -1)).max() <= 1e-5
