@@ -34,9 +34,12 @@ def needs_autograd(H, jump_ops, rho0) -> bool:
         _is_grad_tensor(H) or _is_grad_tensor(rho0) or any(_is_grad_tensor(L) for L in jump_ops))
 
 
-def _accepted(prep) -> int:
-    """The most steps that an instance of the last launch accepted (waits for it)."""
-    return int(prep.bufs['infos'].cpu().numpy()[:, 1].max(initial=0))
+def _counts(prep):
+    """The most steps that an instance of the last launch accepted, and the instances' statuses
+    (host): one read-back, which waits for the launch."""
+    host = prep.bufs['counts'].cpu()
+    B = prep.bufs['status'].shape[0]
+    return int(host.numpy()[1:3 * B:3].max(initial=0)), host[3 * B:]
 
 
 def _solve_taped(integ, lib):
@@ -44,7 +47,7 @@ def _solve_taped(integ, lib):
     records them."""
     prep = integ._prepare_dense(lib, 'small')
     prep.launch()
-    _record(integ, lib, prep, max(_accepted(prep), 1))
+    _record(integ, lib, prep, max(_counts(prep)[0], 1))
     return prep
 
 
@@ -171,8 +174,10 @@ def mesolve_autograd(H, jump_ops, rho0, tsave, *, exp_ops, method, gradient, opt
     # The taped solve's own counts decide whether the tape holds every step: it always runs in
     # FP32, and a plain solve of another precision may take fewer.  (Read here, where the
     # result waits for the solve anyway.)
-    while (taken := _accepted(prep)) > prep.bufs['tape'][0].capacity:
+    taken, status = _counts(prep)
+    while taken > prep.bufs['tape'][0].capacity:
         _record(integ, lib, prep, taken)
         states, expects = _Solve.apply(Ht, rt, *Lts)
+        taken, status = _counts(prep)
     # the rest of the result (shapes, infos, checks) as for any solve
-    return integ._result(states, expects, prep.bufs['infos'], prep.bufs['status'])
+    return integ._result(states, expects, prep.bufs['infos'], status)

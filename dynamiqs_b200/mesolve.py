@@ -473,6 +473,7 @@ class MESolveB200Integrator:
         plan = self.plan
         r_items = plan.rho_items
         is_ket = r_items.shape[-1] == 1 and n > 1
+        counts = torch.empty(4 * B, dtype=torch.int32, device=dev)  # (one read-back gives both)
         bufs = {
             **to_device({
                 **{name: (x, c64) for name, x in operators.items()},
@@ -485,8 +486,9 @@ class MESolveB200Integrator:
             }, dev),
             'states': torch.empty((B, nsave, n, n), dtype=c64, device=dev),
             'expects': torch.empty((B, max(nE, 1), ntsave), dtype=c64, device=dev),
-            'infos': torch.empty((B, 3), dtype=torch.int32, device=dev),
-            'status': torch.empty((B,), dtype=torch.int32, device=dev),
+            'counts': counts,
+            'infos': counts[:3 * B].view(B, 3),
+            'status': counts[3 * B:],
         }
         outs = _lib.Outputs(states=bufs['states'].data_ptr(), expects=bufs['expects'].data_ptr(),
                             infos=bufs['infos'].data_ptr(), status=bufs['status'].data_ptr())
