@@ -274,7 +274,8 @@ def test_result_checks_run_on_the_states_device(monkeypatch):
 @pytest.mark.gpu
 def test_upload_is_not_held_up_by_another_stream(cuda_device):
     """An upload on a busy stream, more than the ring's slots long, waits for that stream; one
-    on an idle stream in another thread meanwhile does not."""
+    of another thread, as long as the ring, is enqueued meanwhile.  (Its copies are not waited
+    for: streams that share a hardware queue wait for one another.)"""
     import threading
 
     import torch
@@ -282,12 +283,19 @@ def test_upload_is_not_held_up_by_another_stream(cuda_device):
     from dynamiqs_b200.upload import to_device
 
     big = np.ones((80 << 20) // 8, np.complex64)
-    small = np.ones((32 << 20) // 8, np.complex64)
-    to_device({'x': (big, torch.complex64)}, cuda_device)  # the page-locked blocks, the threads
+    small = np.ones((24 << 20) // 8, np.complex64)
     busy, idle = torch.cuda.Stream(), torch.cuda.Stream()
+    # every block that the uploads will take, device and page-locked, is there before the kernel
+    # starts: an allocation may wait for the device
+    torch.cuda.empty_cache()
+    rings = [torch.empty(24 << 20, dtype=torch.uint8, pin_memory=True) for _ in range(2)]
+    del rings
+    for stream, a in ((busy, big), (idle, small)):
+        with torch.cuda.stream(stream):
+            to_device({'x': (a, torch.complex64)}, cuda_device)
     torch.cuda.synchronize()
     with torch.cuda.stream(busy):
-        torch.cuda._sleep(3_000_000_000)  # about 1.5 s, then it ends
+        torch.cuda._sleep(6_000_000_000)  # about 3 s, then it ends
         end = torch.cuda.Event()
         end.record()
 
@@ -300,10 +308,10 @@ def test_upload_is_not_held_up_by_another_stream(cuda_device):
     time.sleep(0.3)  # the first upload fills its ring and waits
     with torch.cuda.stream(idle):
         out = to_device({'x': (small, torch.complex64)}, cuda_device)['x']
+        enqueued_first = not end.query()
         idle.synchronize()
-        done_first = not end.query()
     other.join()
-    assert done_first and bool((out == 1).all())
+    assert enqueued_first and bool((out == 1).all())
 
 
 def test_upload_copies_without_its_threads():
