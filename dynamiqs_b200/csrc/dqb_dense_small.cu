@@ -1090,7 +1090,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) mesolve_adjoint_kernel(AdjAr
 // X Zs = (Zs X)^+.  Other instances are marked and left to mesolve_adjoint_kernel.
 // Measured (one B200): driven Kerr, n = 30, one jump, 64 instances: 0.59 against 2.43 ms.
 
-// KR: jump operators that it takes at most.  tape_np: row length of the tape's states.
+// KR: jump operators that it takes at most: two up to n = 32 (Bands has masks for two), one up to
+// 48 (12 matrices of 18.8 KB fill the shared memory).  tape_np: row length of the tape's states.
 template <int NP, int KR>
 __global__ void __launch_bounds__(kSmallThreads, NP <= 16 ? 2 : 1) mesolve_adjoint_band_kernel(AdjArgs A, int tape_np,
                                                                                               int* marks) {

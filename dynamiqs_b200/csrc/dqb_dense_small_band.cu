@@ -21,7 +21,7 @@
 // tiles, thread (ty, tx) owns element (ty, tx) of each of the R (R + 1) / 2 upper tiles and
 // keeps k_2..k_7 of them in registers (120 of a thread's 255 at n = 64) and y and k_1 in
 // shared memory, where the rest of the registers is wanted for the right-hand side (with
-// all of them in registers the spills went to L2: 20.0 against 17.1 ms below).  Shared
+// all of them in registers the spills went to L2: 20.0 against 17.1 ms then).  Shared
 // memory also holds the stage input X, whole (the stencil reads both triangles; the owner of
 // (i, j) also writes conj(X) at (j, i)), in two buffers, so that a right-hand side costs one
 // barrier.  A row (column) coefficient is read once per tile row (column) and used on all
@@ -30,10 +30,10 @@
 // alike, which needs no barrier.  Two warps per scheduler issue in 40% of the cycles; the
 // rest are fixed latencies, shared-memory waits and instruction fetch.
 //
-// Measured (one B200): driven Kerr, n = 64, two jumps, 1024 instances, t = 1.6: 16.9 ms
-// against 153.4 ms for the product kernel; n = 21, one jump, 1000 instances: 1.45 against
+// Measured (one B200): driven Kerr, n = 64, two jumps, 1024 instances, t = 1.6: 16.1 ms
+// against 153.4 ms for the product kernel; n = 21, one jump, 1000 instances: 1.5 against
 // 5.31 ms; n = 8, 2000 instances: 0.42 against 2.28 ms; one n = 16 oscillator with 101 saves:
-// 0.27 against 0.72 ms (0.38 with one diagonal per pass and registers for four CTAs per SM).
+// 0.25 against 0.72 ms (0.38 with one diagonal per pass and registers for four CTAs per SM).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -44,6 +44,8 @@
 namespace dqb {
 namespace band {
 
+// What the packed offsets (offset_of) and the tables hold; at eight the kernel is still 1.6
+// (n = 32) to 3.3 (n = 8) times as fast as the products, eight jump operators 5 to 7 times.
 constexpr int kMaxH = 8;   // nonzero diagonals of Hnh
 constexpr int kMaxK = 8;   // jump operators
 constexpr int kMaxL = 8;   // nonzero diagonals of all jump operators together

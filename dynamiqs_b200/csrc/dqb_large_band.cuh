@@ -23,6 +23,8 @@
 // hermitian-half kernels read it.
 #pragma once
 
+// What the records hold; at eight diagonals of Hnh, no jump, the stencil is still 1.8 (n = 100,
+// 32 instances) to 3.9 (n = 256, 32) times as fast as the products.
 constexpr int kBandMaxH = 8;  // nonzero diagonals of Hnh
 constexpr int kBandMaxL = 8;  // nonzero diagonals of the jump operators together
 constexpr int kBandMaxK = 8;  // jump operators
